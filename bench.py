@@ -33,7 +33,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.join(ROOT, "gpu-cgfd3d-dynamic_b200")
 sys.path.insert(0, PKG)
 
-BYTES_PER_POINT_STEP = 768          # algorithmic HBM traffic of one point and step (FP32)
+BYTES_PER_POINT_STEP = 624          # algorithmic HBM traffic of one point and step (FP32)
 FALLBACK_HBM_GBS = 6650.0
 
 

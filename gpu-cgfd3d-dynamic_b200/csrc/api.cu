@@ -300,7 +300,7 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
   // the fault kernels' arguments of one stage
   auto stage_fargs = [&](int stage, FaultArgs *fa) {
     const int idir = (kPairs[ip][0] + stage) % 2, jdir = (kPairs[ip][1] + stage) % 2, kdir = (kPairs[ip][2] + stage) % 2;
-    const int mode = stage == 0 ? RK_FIRST : (stage == 3 ? RK_LAST : RK_MID);
+    const int mode = stage;   // RK_FIRST .. RK_LAST
     const int Lcur = stage == 0 ? LP : (stage == 2 ? LB : LA);
     const int Lout = stage == 0 ? LA : (stage == 1 ? LB : (stage == 2 ? LA : -1));
     const real ca = stage < 3 ? kRkA[stage] * s->dt : RL(0.0), cb = kRkB[stage] * s->dt;
@@ -355,7 +355,7 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
   const int nfa = stage_fargs(0, fargs);
   for (int stage = 0; stage < 4; stage++) {
     const int idir = (kPairs[ip][0] + stage) % 2, jdir = (kPairs[ip][1] + stage) % 2, kdir = (kPairs[ip][2] + stage) % 2;
-    const int mode = stage == 0 ? RK_FIRST : (stage == 3 ? RK_LAST : RK_MID);
+    const int mode = stage;   // RK_FIRST .. RK_LAST
     const int Lcur = stage == 0 ? LP : (stage == 2 ? LB : LA);
     const int Lout = stage == 0 ? LA : (stage == 1 ? LB : (stage == 2 ? LA : -1));
     const real ca = stage < 3 ? kRkA[stage] * s->dt : RL(0.0), cb = kRkB[stage] * s->dt;

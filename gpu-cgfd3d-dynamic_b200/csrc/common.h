@@ -12,7 +12,8 @@
 // 9 components (Vx,Vy,Vz,Txx,Tyy,Tzz,Tyz,Txz,Txy) of scmp points as two
 // arrays of 16-byte groups (Vx Vy Vz Txx | Tyy Tzz Tyz Txz) and one of Txy,
 // so that a stencil tap reads all nine with three loads (Grid::w); four levels
-// P (time n), A and B (ping-pong stage inputs) and E (time n+1 accumulator)
+// P (time n), A and B (ping-pong stage inputs) and E (the second stage's
+// V, then time n+1: RK_FIRST in ops.cuh)
 // replace the reference's pre/tmp/rhs/end, because each fused stage writes
 // its output level directly instead of a separate rhs array.
 #pragma once
@@ -103,7 +104,7 @@ struct PmlFaceDev {
   const real *A, *B, *D;   // per layer along the normal
   // auxiliary-field levels used by one stage (9*siz floats each, grouped
   // like a wavefield level with siz points per component): stage input,
-  // time-n level, next-stage output, end accumulator
+  // time-n level, next-stage output, fourth level (V, then time n+1)
   const real *acur, *apre;
   real *aout, *aend;
 };

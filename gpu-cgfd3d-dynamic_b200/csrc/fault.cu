@@ -77,28 +77,30 @@ __device__ __forceinline__ void odd_image(real v[7], int nf) {
   }
 }
 
-// stage update of N values; every level read is issued before the first
-// store (the compiler cannot prove that the levels do not alias, and
-// interleaved load / store pairs cost one memory round trip each)
+// RK stage update of N values (see RK_FIRST in ops.cuh); every level read
+// is issued before the first store (the compiler cannot prove that the
+// levels do not alias, and interleaved load / store pairs cost one memory
+// round trip each)
 template <int N>
 __device__ __forceinline__ void rk_put_n(int mode, real ca, real cb, const real *cur, const real *pre,
                                          real *out, real *end, const long o[N], const real h[N]) {
   real u[N], e[N];
+#pragma unroll
+  for (int n = 0; n < N; n++) {
+    if (mode != RK_THIRD) u[n] = cur[o[n]];
+    if (mode != RK_FIRST) e[n] = mode == RK_LAST ? end[o[n]] : pre[o[n]];
+  }
   if (mode == RK_FIRST) {
 #pragma unroll
-    for (int n = 0; n < N; n++) u[n] = cur[o[n]];
+    for (int n = 0; n < N; n++) out[o[n]] = rk_out(u[n], ca * h[n]);
+  } else if (mode == RK_LAST) {
 #pragma unroll
-    for (int n = 0; n < N; n++) { out[o[n]] = u[n] + ca * h[n]; end[o[n]] = u[n] + cb * h[n]; }
+    for (int n = 0; n < N; n++) end[o[n]] = rk_end(e[n], u[n], cb * h[n]);
   } else {
 #pragma unroll
     for (int n = 0; n < N; n++) {
-      if (mode == RK_MID) u[n] = pre[o[n]];
-      e[n] = end[o[n]];
-    }
-#pragma unroll
-    for (int n = 0; n < N; n++) {
-      if (mode == RK_MID) out[o[n]] = u[n] + ca * h[n];
-      end[o[n]] = e[n] + cb * h[n];
+      out[o[n]] = rk_out(e[n], ca * h[n]);
+      if (mode == RK_SECOND) end[o[n]] = rk_v(e[n], u[n], ca * h[n]);
     }
   }
 }
@@ -735,12 +737,11 @@ __device__ __forceinline__ void lev9(const real *w, long sc, long p, real v[9]) 
   v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
   v[8] = w[8 * sc + p];
 }
-// level value + c * h at point p, whole 16-byte groups
-__device__ __forceinline__ void put9(real *w, long sc, long p, const real v[9], real c, const real h[9]) {
-  reinterpret_cast<real4 *>(w)[p] = make_real4(v[0] + c * h[0], v[1] + c * h[1], v[2] + c * h[2], v[3] + c * h[3]);
-  reinterpret_cast<real4 *>(w + 4 * sc)[p] =
-      make_real4(v[4] + c * h[4], v[5] + c * h[5], v[6] + c * h[6], v[7] + c * h[7]);
-  w[8 * sc + p] = v[8] + c * h[8];
+// nine components to point p of a level, whole 16-byte groups
+__device__ __forceinline__ void put9(real *w, long sc, long p, const real v[9]) {
+  reinterpret_cast<real4 *>(w)[p] = make_real4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<real4 *>(w + 4 * sc)[p] = make_real4(v[4], v[5], v[6], v[7]);
+  w[8 * sc + p] = v[8];
 }
 
 // the six volume points i0-3..i0+3 (not i0) of split nodes, one thread per
@@ -756,16 +757,22 @@ __global__ void __launch_bounds__(192) k_fault_slab(const FaultArgs a) {
   slab_velocity(a, j, k, s, h);
   slab_stress(a, j, k, s, h + 3);
   const long q = g.at(a.F.i0 + s, j + NG, k + NG), sc = g.scmp;
-  real u[9], e[9];
-  if (a.mode == RK_FIRST) {
-    lev9(a.wcur, sc, q, u);
-    put9(a.wout, sc, q, u, a.ca, h);
-    put9(a.wend, sc, q, u, a.cb, h);
-  } else {
-    if (a.mode == RK_MID) lev9(a.wpre, sc, q, u);
-    lev9(a.wend, sc, q, e);
-    if (a.mode == RK_MID) put9(a.wout, sc, q, u, a.ca, h);
-    put9(a.wend, sc, q, e, a.cb, h);
+  real u[9], e[9], r[9];
+  if (a.mode != RK_THIRD) lev9(a.wcur, sc, q, u);
+  if (a.mode != RK_FIRST) lev9(a.mode == RK_LAST ? a.wend : a.wpre, sc, q, e);
+  if (a.mode == RK_LAST) {
+#pragma unroll
+    for (int c = 0; c < 9; c++) r[c] = rk_end(e[c], u[c], a.cb * h[c]);
+    put9(a.wend, sc, q, r);
+    return;
+  }
+#pragma unroll
+  for (int c = 0; c < 9; c++) r[c] = rk_out(a.mode == RK_FIRST ? u[c] : e[c], a.ca * h[c]);
+  put9(a.wout, sc, q, r);
+  if (a.mode == RK_SECOND) {
+#pragma unroll
+    for (int c = 0; c < 9; c++) r[c] = rk_v(e[c], u[c], a.ca * h[c]);
+    put9(a.wend, sc, q, r);
   }
 }
 

@@ -34,7 +34,7 @@
 // normal d reuses direction d's contribution.
 //
 // Roofline: HBM-bound.  Algorithmic traffic per point and step is
-// 192 floats = 768 B (21+18, 39+18, 39+18, 30+9 floats over the 4 stages).
+// 156 floats = 624 B (21+9, 30+18, 30+9, 30+9 floats over the 4 stages).
 #include <cuda_runtime.h>
 
 #include "ops.cuh"
@@ -168,12 +168,45 @@ __device__ __forceinline__ void ld9(const real *w, long sc, long p, real v[9], b
   v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
   v[8] = ro ? __ldg(w + 8 * sc + p) : w[8 * sc + p];
 }
-// level value + k * h at point p of level w
-__device__ __forceinline__ void st9(real *w, long sc, long p, const real v[9], real k, const real h[9]) {
-  reinterpret_cast<real4 *>(w)[p] = make_real4(v[0] + k * h[0], v[1] + k * h[1], v[2] + k * h[2], v[3] + k * h[3]);
-  reinterpret_cast<real4 *>(w + 4 * sc)[p] =
-      make_real4(v[4] + k * h[4], v[5] + k * h[5], v[6] + k * h[6], v[7] + k * h[7]);
-  w[8 * sc + p] = v[8] + k * h[8];
+// the nine components of point p of level w
+__device__ __forceinline__ void st9(real *w, long sc, long p, const real v[9]) {
+  reinterpret_cast<real4 *>(w)[p] = make_real4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<real4 *>(w + 4 * sc)[p] = make_real4(v[4], v[5], v[6], v[7]);
+  w[8 * sc + p] = v[8];
+}
+
+// RK stage update (see RK_FIRST in ops.cuh) of nine components at point p of
+// levels with sc points per component: cur holds the stage input's values,
+// h their rates.  All reads of the levels are issued before the first
+// store: the compiler cannot prove that the levels do not alias, and
+// interleaved load / store pairs would cost one memory round trip per
+// component.
+template <int MODE>
+__device__ __forceinline__ void rk_point(const real *pre, real *out, real *end, long sc, long p, real ca, real cb,
+                                         const real cur[9], const real h[9]) {
+  real r[9];
+  if (MODE == RK_FIRST) {
+#pragma unroll
+    for (int c = 0; c < 9; c++) r[c] = rk_out(cur[c], ca * h[c]);
+    st9(out, sc, p, r);
+  } else if (MODE == RK_LAST) {
+    real v[9];
+    ld9(end, sc, p, v, false);
+#pragma unroll
+    for (int c = 0; c < 9; c++) r[c] = rk_end(v[c], cur[c], cb * h[c]);
+    st9(end, sc, p, r);
+  } else {
+    real u0[9];
+    ld9(pre, sc, p, u0, true);
+#pragma unroll
+    for (int c = 0; c < 9; c++) r[c] = rk_out(u0[c], ca * h[c]);
+    st9(out, sc, p, r);
+    if (MODE == RK_SECOND) {
+#pragma unroll
+      for (int c = 0; c < 9; c++) r[c] = rk_v(u0[c], cur[c], ca * h[c]);
+      st9(end, sc, p, r);
+    }
+  }
 }
 // L2 prefetch of the auxiliary-field lines that pml_face reads at (I, J, K)
 template <int MODE>
@@ -181,7 +214,7 @@ __device__ __forceinline__ void pml_prefetch(const PmlFaceDev &P, int I, int J, 
   const int li = I - P.i1, lj = J - P.j1, lk = K - P.k1;
   if (li < 0 || li >= P.fni || lj < 0 || lj >= P.fnj || lk < 0 || lk >= P.fnk) return;
   const long pa = li + (long)lj * P.fni + (long)lk * P.fni * P.fnj, sz = P.siz;
-  const real *lv[3] = { P.acur, MODE == RK_MID ? P.apre : nullptr, MODE != RK_FIRST ? P.aend : nullptr };
+  const real *lv[3] = { P.acur, rk_reads_pre(MODE) ? P.apre : nullptr, MODE == RK_LAST ? P.aend : nullptr };
 #pragma unroll
   for (int l = 0; l < 3; l++) {
     if (!lv[l]) continue;
@@ -227,36 +260,13 @@ __device__ __forceinline__ void pml_face(const VolArgs &a, const PmlFaceDev &P, 
 #pragma unroll
     for (int c = TXX; c <= TXY; c++) { corr[c] += (cB - 1.0f) * q[c]; ar[c] += cD * q[c]; }
   }
-  // auxiliary RK update; level reads first (see rk_update)
-  if (MODE == RK_FIRST) {
-    st9(P.aout, P.siz, pa, ac, a.ca, ar);
-    st9(P.aend, P.siz, pa, ac, a.cb, ar);
-  } else {
-    real pv[9], ev[9];
-    if (MODE == RK_MID) ld9(P.apre, P.siz, pa, pv, true);
-    ld9(P.aend, P.siz, pa, ev, false);
-    if (MODE == RK_MID) st9(P.aout, P.siz, pa, pv, a.ca, ar);
-    st9(P.aend, P.siz, pa, ev, a.cb, ar);
-  }
+  rk_point<MODE>(P.apre, P.aout, P.aend, P.siz, pa, a.ca, a.cb, ac, ar);
 }
 
-// RK stage update of the nine components at p.  All reads of the levels
-// are issued before the first store: the compiler cannot prove that out
-// and end do not alias, and interleaved load / store pairs would cost one
-// memory round trip per component.
+// RK stage update of the wavefield at p
 template <int MODE>
 __device__ __forceinline__ void rk_update(const VolArgs &a, long p, const real v0[9], const real h[9]) {
-  const long sc = a.g.scmp;
-  if (MODE == RK_FIRST) {
-    st9(a.out, sc, p, v0, a.ca, h);
-    st9(a.end, sc, p, v0, a.cb, h);
-  } else {
-    real pv[9], ev[9];
-    if (MODE == RK_MID) ld9(a.pre, sc, p, pv, true);
-    ld9(a.end, sc, p, ev, false);
-    if (MODE == RK_MID) st9(a.out, sc, p, pv, a.ca, h);
-    st9(a.end, sc, p, ev, a.cb, h);
-  }
+  rk_point<MODE>(a.pre, a.out, a.end, a.g.scmp, p, a.ca, a.cb, v0, h);
 }
 
 // kernel kinds: the interior box (no boundary logic), slabs that only PML
@@ -357,12 +367,12 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
   const long sc = g.scmp;
 #if CGFD_PREFETCH
   if (MODE != RK_FIRST) {
-    // the RK update reads the time-n level and the accumulator last: ask
-    // L2 for their lines now, so that those reads wait on L2, not DRAM
-    const real *q[6] = { a.end + 4 * p, a.end + 4 * sc + 4 * p, a.end + 8 * sc + p,
-                          a.pre + 4 * p, a.pre + 4 * sc + 4 * p, a.pre + 8 * sc + p };
-#pragma unroll
-    for (int n = 0; n < (MODE == RK_MID ? 6 : 3); n++) asm volatile("prefetch.global.L2 [%0];" ::"l"(q[n]));
+    // the RK update reads the time-n level (or, last, the V level) at its
+    // end: ask L2 for its lines now, so that those reads wait on L2, not DRAM
+    const real *l = MODE == RK_LAST ? a.end : a.pre;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(l + 4 * p));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(l + 4 * sc + 4 * p));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(l + 8 * sc + p));
   }
 #if CGFD_AHEAD > 0
   if (KIND == INTERIOR) {
@@ -568,7 +578,8 @@ void launch4(const VolArgs &a, int mode, cudaStream_t st) {
     grd = dim3(B.nbx, a.ychunk, (B.k1 - B.k0 + 1) * nchunks);
   }
   if (mode == RK_FIRST) k_volume<ID, JD, KD, RK_FIRST, KIND><<<grd, blk, 0, st>>>(a);
-  else if (mode == RK_MID) k_volume<ID, JD, KD, RK_MID, KIND><<<grd, blk, 0, st>>>(a);
+  else if (mode == RK_SECOND) k_volume<ID, JD, KD, RK_SECOND, KIND><<<grd, blk, 0, st>>>(a);
+  else if (mode == RK_THIRD) k_volume<ID, JD, KD, RK_THIRD, KIND><<<grd, blk, 0, st>>>(a);
   else k_volume<ID, JD, KD, RK_LAST, KIND><<<grd, blk, 0, st>>>(a);
 }
 
@@ -589,7 +600,7 @@ void launch_kind(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaS
 }  // namespace
 
 // This file is compiled once per kernel kind (CGFD_VOLUME_KIND = 0..7, set
-// by the build) so that the 24 instantiations of each kind build in
+// by the build) so that the 32 instantiations of each kind build in
 // parallel; unit 0 also holds the host helpers.
 #ifndef CGFD_VOLUME_KIND
 #define CGFD_VOLUME_KIND 0
