@@ -632,7 +632,7 @@ int cgfd_create(const cgfd_config *cfg, cgfd_solver **out) {
 static int build_graphs(cgfd_solver *s);
 
 
-// Autotuner of the interior kernel's y chunk (the number of 8-row tiles whose
+// Autotuner of the interior kernel's y chunk (the number of kTileY-row tiles whose
 // blocks march up z together, which sets how much of L2 the stencil planes
 // take): the first stage's interior launch is timed for a few chunk sizes
 // on the solver's state at upload, which is all zero, so the launches write
@@ -653,7 +653,7 @@ static cudaError_t tune_ychunk(cgfd_solver *s) {
     auto f = g_tune.find(key);
     if (f != g_tune.end()) { s->ychunk = f->second; return cudaSuccess; }
   }
-  const int ntiles = (key[2] + 7) / 8, ip = s->it % 8, it = s->it;
+  const int ntiles = (key[2] + kTileY - 1) / kTileY, ip = s->it % 8, it = s->it;
   VolArgs v{};
   v.g = s->g; v.cur = s->w[slot(LP, it)]; v.pre = v.cur; v.out = s->w[slot(LA, it)]; v.end = s->w[slot(LE, it)];
   v.coef = s->coef; v.free_mat = s->free_mat;
@@ -667,7 +667,7 @@ static cudaError_t tune_ychunk(cgfd_solver *s) {
   int best = s->ychunk;
   float best_ms = 1e30f;
   std::vector<int> cand;
-  for (int c : { 8, 16, 32, 64, ntiles }) {
+  for (int c : { 16, 32, 64, 128, ntiles }) {
     c = std::max(1, std::min(c, ntiles));
     if (std::find(cand.begin(), cand.end(), c) == cand.end()) cand.push_back(c);
   }
@@ -813,19 +813,24 @@ int cgfd_upload(const cgfd_setup *su, cgfd_solver **out) {
       b[0] = i0; b[1] = i1; b[2] = j0; b[3] = j1; b[4] = k0; b[5] = k1;
     };
     const int ni = g.ni, nj = g.nj, nk = g.nk;
-    // the interior box is a whole number of 32-point tiles wide in x; the
-    // columns left over (fewer than 32) join the right x PML slab, not a last
-    // tile of each row whose warps would have only those few lanes at work
-    // (unless a fault's neighbourhood reaches them: the fault kernels may
-    // start beside the PML kernels only away from their boxes).  The y and z
-    // PML slabs and the surface rows over the interior box's x extent are
-    // cut the same way, their leftover columns going to the generic edge and
-    // shell kernels
+    // up to kMaxLeftover columns beyond a whole number of 32-point tiles join
+    // the right x PML slab instead of making a last tile of each row whose
+    // warps have only those few lanes at work (unless a fault's
+    // neighbourhood reaches them: the fault kernels may start beside the PML
+    // kernels only away from their boxes).  The y and z PML slabs and the
+    // surface rows over the interior box's x extent are cut the same way,
+    // their leftover columns going to the generic edge and shell kernels.
+    // The PML kernels take about 1.8 times the interior kernel's time per
+    // point, so more columns stay where they are: measured per step, all
+    // joining / staying: 6 columns (240 wide) 2.754 / 2.814 ms, 14 (100 wide)
+    // 0.512 / 0.507, 15 (101) 0.457 / 0.437, 24 (120) 0.518 / 0.488, 30 (200)
+    // 2.339 / 2.221.
+    constexpr int kMaxLeftover = 8;
     int iha = ihi;
     {
       const int w = ihi - ilo + 1, wa = w / 32 * 32;
       const char *at = std::getenv("CGFD_ALIGN_TILES");
-      bool split = wa > 0 && wa < w && !(at && at[0] == '0');
+      bool split = wa > 0 && wa < w && w - wa <= kMaxLeftover && !(at && at[0] == '0');
       for (auto &F : s->faults)
         if (F.d.i0 - NG + 6 >= ilo + wa && F.d.i0 - NG - 6 <= ihi) split = false;
       if (split) iha = ilo + wa - 1;
@@ -902,17 +907,17 @@ int cgfd_upload(const cgfd_setup *su, cgfd_solver **out) {
     if (pq && pq[0] == '0') s->post_early = false;
     const char *pk = std::getenv("CGFD_PACK");
     if (pk && pk[0] == '0') s->pack = false;
-    // y tiles (8 rows) per interior chunk: the z window of a chunk, about 8
+    // y tiles (kTileY rows) per interior chunk: the z window of a chunk, about 8
     // planes of the stage input (36 B a point), should take at most ~24 MB
     // of the 126 MB L2, which also carries the streamed arrays (measured:
-    // 1200x600x400 best at 16-24 tiles, 600x300x240 at its whole plane)
+    // 1200x600x400 best at 128-192 rows, 600x300x240 at its whole plane)
     {
-      const long row_bytes = (long)std::max(1, ihi - ilo + 1) * 8 * 36;
+      const long row_bytes = (long)std::max(1, ihi - ilo + 1) * kTileY * 36;
       s->ychunk = (int)std::max(4L, (24L << 20) / (8 * row_bytes));
     }
     const char *yc = std::getenv("CGFD_INTERIOR_YCHUNK");
     if (yc && std::atoi(yc) > 0) s->ychunk = std::atoi(yc);
-    s->ychunk = std::min(s->ychunk, std::max(1, (jhi - jlo + 8) / 8));
+    s->ychunk = std::min(s->ychunk, std::max(1, (jhi - jlo + kTileY) / kTileY));
     // points one interior launch / one volume stage updates: the split-node
     // slabs belong to the fault kernels
     long long nint = (long long)std::max(0, iha - ilo + 1) * std::max(0, jhi - jlo + 1) * std::max(0, khi - klo + 1);

@@ -43,8 +43,7 @@ namespace cgfd {
 
 namespace {
 
-constexpr int BX = 32, BY = 8;
-
+constexpr int BX = kTileX, BY = kTileY;
 
 // conservative traction J * (e . sigma_row) at point q for metric row d
 // (0: xi, 1: eta, 2: zeta), all three stress rows (xx,xy,xz), (xy,yy,yz),
@@ -74,12 +73,76 @@ __device__ __forceinline__ Taps taps_at(const real *w, long sc, long p) {
   T.t = w + 8 * sc + p;
   return T;
 }
+// Nine components of a point as they lie in memory: the pairs (Vx Vy) (Vz
+// Txx) (Tyy Tzz) (Tyz Txz) and Txy.  The stencil sums run on pairs: on
+// sm_100 one fma.rn.f32x2 does two multiply-adds, each rounded as the
+// scalar one, so the 27 derivatives of a point take 75 instructions instead
+// of 135 (interior launch of 30.0 M points with waves everywhere, where the
+// GPU sits at its 1000 W cap: 1.089 -> 1.058 ms; from 16-24 bytes of spills to
+// none at 64 registers).
+#ifdef CGFD_FP64
+typedef double2 real2;
+__device__ __forceinline__ real2 mul2(real c, real2 x) { return make_double2(c * x.x, c * x.y); }
+__device__ __forceinline__ real2 fma2(real c, real2 x, real2 y) { return make_double2(fma(c, x.x, y.x), fma(c, x.y, y.y)); }
+__device__ __forceinline__ void split2(real2 v, real &x, real &y) { x = v.x; y = v.y; }
+__device__ __forceinline__ void ldg4(const real4 *q, real2 &x, real2 &y) {
+  x = ::__ldg(reinterpret_cast<const double2 *>(q));
+  y = ::__ldg(reinterpret_cast<const double2 *>(q) + 1);
+}
+#else
+typedef unsigned long long real2;
+__device__ __forceinline__ real2 pack2(real x, real y) {
+  real2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void split2(real2 v, real &x, real &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ real2 mul2(real c, real2 x) {
+  real2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(c, c)), "l"(x));
+  return r;
+}
+__device__ __forceinline__ real2 fma2(real c, real2 x, real2 y) {
+  real2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack2(c, c)), "l"(x), "l"(y));
+  return r;
+}
+__device__ __forceinline__ void ldg4(const real4 *q, real2 &x, real2 &y) {
+  const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(q));
+  x = v.x;
+  y = v.y;
+}
+#endif
+struct V9 {
+  real2 p[4];
+  real t;
+};
+__device__ __forceinline__ void unpack9(const V9 &v, real d[9]) {
+#pragma unroll
+  for (int n = 0; n < 4; n++) split2(v.p[n], d[2 * n], d[2 * n + 1]);
+  d[8] = v.t;
+}
+__device__ __forceinline__ V9 mul9(real c, const V9 &x) {
+  V9 r;
+#pragma unroll
+  for (int n = 0; n < 4; n++) r.p[n] = mul2(c, x.p[n]);
+  r.t = c * x.t;
+  return r;
+}
+__device__ __forceinline__ V9 fma9(real c, const V9 &x, const V9 &y) {
+  V9 r;
+#pragma unroll
+  for (int n = 0; n < 4; n++) r.p[n] = fma2(c, x.p[n], y.p[n]);
+  r.t = fma(c, x.t, y.t);
+  return r;
+}
 // the nine components of the point o points away
-__device__ __forceinline__ void ld9(const Taps &T, int o, real v[9]) {
-  const real4 x = __ldg(T.a + o), y = __ldg(T.b + o);
-  v[VX] = x.x; v[VY] = x.y; v[VZ] = x.z; v[TXX] = x.w;
-  v[TYY] = y.x; v[TZZ] = y.y; v[TYZ] = y.z; v[TXZ] = y.w;
-  v[TXY] = __ldg(T.t + o);
+__device__ __forceinline__ V9 tap9(const Taps &T, int o) {
+  V9 v;
+  ldg4(T.a + o, v.p[0], v.p[1]);
+  ldg4(T.b + o, v.p[2], v.p[3]);
+  v.t = __ldg(T.t + o);
+  return v;
 }
 
 template <int F>
@@ -108,55 +171,52 @@ __device__ __forceinline__ void rhs_dir(const real D[9], const real e[3], real l
   r[TYZ] = mu * (e[2] * D[VY] + e[1] * D[VZ]);
 }
 
-// one-sided DRP derivatives of the nine components, the centre sample v0
-// known; off[n] are the offsets of the 4 other taps in table order
-// (F: -1, 0, 1, 2, 3; B: -3, -2, -1, 0, 1 with the centre at n = 1 / 3).
-// Each tap's nine components come in one go; the sums keep the order of
-// the coefficient table.
+// one-sided DRP derivatives of the nine components in table order (F:
+// offsets -1, 0, 1, 2, 3; B: -3, -2, -1, 0, 1), the centre sample v0 known;
+// off[n] are the offsets of the other four taps
 template <int F>
-__device__ __forceinline__ void derivs(const Taps &T, const real v0[9], const int off[4], real D[9]) {
-  real t[9];
-  ld9(T, off[0], t);
-#pragma unroll
-  for (int c = 0; c < 9; c++) D[c] = (F ? kC1 : kC5) * t[c];
-  if (F) {
-#pragma unroll
-    for (int c = 0; c < 9; c++) D[c] += kC2 * v0[c];
-  }
-  ld9(T, off[1], t);
-#pragma unroll
-  for (int c = 0; c < 9; c++) D[c] += (F ? kC3 : kC4) * t[c];
-  ld9(T, off[2], t);
-#pragma unroll
-  for (int c = 0; c < 9; c++) D[c] += (F ? kC4 : kC3) * t[c];
-  if (!F) {
-#pragma unroll
-    for (int c = 0; c < 9; c++) D[c] += kC2 * v0[c];
-  }
-  ld9(T, off[3], t);
-#pragma unroll
-  for (int c = 0; c < 9; c++) D[c] = F ? D[c] + kC5 * t[c] : -(D[c] + kC1 * t[c]);
+__device__ __forceinline__ void derivs(const Taps &T, const V9 &v0, const int off[4], real D[9]) {
+  V9 r = mul9(wdrp<F>(0), tap9(T, off[0]));
+  if (F) r = fma9(wdrp<F>(1), v0, r);
+  r = fma9(wdrp<F>(F ? 2 : 1), tap9(T, off[1]), r);
+  r = fma9(wdrp<F>(F ? 3 : 2), tap9(T, off[2]), r);
+  if (!F) r = fma9(wdrp<F>(3), v0, r);
+  unpack9(fma9(wdrp<F>(4), tap9(T, off[3]), r), D);
 }
 
-// Accumulate one direction's derivatives straight into the velocity
-// gradient G[c][b] = dV_c/dx_b and the momentum sums
+// Accumulate one direction's derivatives straight into the strain rates
+// E = (xx, yy, zz, yz, xz, xy), the shear ones as the sums dV_b/dx_c +
+// dV_c/dx_b that Hooke's law needs, and the momentum sums
 // s_r = sum_a e_a . d(sigma_row r)/dxi_a.
-template <int F>
-__device__ __forceinline__ void acc_dir(const Taps &T, const real v0[9], const int off[4], const real ea[3],
-                                        real G[3][3], real s[3]) {
-  real D[9];
-  derivs<F>(T, v0, off, D);
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const real d = D[VX + c];
-    G[c][0] += ea[0] * d; G[c][1] += ea[1] * d; G[c][2] += ea[2] * d;
-  }
+__device__ __forceinline__ void accumulate(const real D[9], const real ea[3], real E[6], real s[3]) {
+  E[0] += ea[0] * D[VX];
+  E[1] += ea[1] * D[VY];
+  E[2] += ea[2] * D[VZ];
+  E[3] += ea[2] * D[VY]; E[3] += ea[1] * D[VZ];
+  E[4] += ea[2] * D[VX]; E[4] += ea[0] * D[VZ];
+  E[5] += ea[1] * D[VX]; E[5] += ea[0] * D[VY];
   s[0] += ea[0] * D[TXX];
   s[1] += ea[1] * D[TYY];
   s[2] += ea[2] * D[TZZ];
   s[1] += ea[2] * D[TYZ]; s[2] += ea[1] * D[TYZ];
   s[0] += ea[2] * D[TXZ]; s[2] += ea[0] * D[TXZ];
   s[0] += ea[1] * D[TXY]; s[1] += ea[0] * D[TXY];
+}
+template <int F>
+__device__ __forceinline__ void acc_dir(const Taps &T, const V9 &v0, const int off[4], const real ea[3],
+                                        real E[6], real s[3]) {
+  real D[9];
+  derivs<F>(T, v0, off, D);
+  accumulate(D, ea, E, s);
+}
+// rates of the nine components from the accumulated sums
+__device__ __forceinline__ void rates(const real E[6], const real s[3], real lam, real mu, real slw, real h[9]) {
+  const real l2m = lam + 2.0f * mu;
+  h[VX] = slw * s[0]; h[VY] = slw * s[1]; h[VZ] = slw * s[2];
+  h[TXX] = l2m * E[0] + lam * (E[1] + E[2]);
+  h[TYY] = l2m * E[1] + lam * (E[0] + E[2]);
+  h[TZZ] = l2m * E[2] + lam * (E[0] + E[1]);
+  h[TYZ] = mu * E[3]; h[TXZ] = mu * E[4]; h[TXY] = mu * E[5];
 }
 
 // the nine components of point p of a level in the grouped layout with
@@ -208,6 +268,12 @@ __device__ __forceinline__ void rk_point(const real *pre, real *out, real *end, 
     }
   }
 }
+// L2 prefetch of the lines of point p of a level
+__device__ __forceinline__ void prefetch9(const real *w, long sc, long p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(w + 4 * p));
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(w + 4 * sc + 4 * p));
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(w + 8 * sc + p));
+}
 // L2 prefetch of the auxiliary-field lines that pml_face reads at (I, J, K)
 template <int MODE>
 __device__ __forceinline__ void pml_prefetch(const PmlFaceDev &P, int I, int J, int K) {
@@ -218,9 +284,7 @@ __device__ __forceinline__ void pml_prefetch(const PmlFaceDev &P, int I, int J, 
 #pragma unroll
   for (int l = 0; l < 3; l++) {
     if (!lv[l]) continue;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(lv[l] + 4 * pa));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(lv[l] + 4 * sz + 4 * pa));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(lv[l] + 8 * sz + pa));
+    prefetch9(lv[l], sz, pa);
   }
 }
 
@@ -320,6 +384,22 @@ __device__ __forceinline__ bool locate_interior(const VolArgs &a, int &i, int &j
   return i <= B.i1 && j <= B.j1;
 }
 
+// points that another kernel updates: the split-node slabs (i0-3..i0+3 of
+// unwelded nodes) belong to the fault kernels; with defer_i0 the fault
+// planes go to the PLANE launch
+template <int KIND>
+__device__ __forceinline__ bool other_kernels_point(const VolArgs &a, int I, int J, int K) {
+  for (int f = 0; f < a.nfault; f++) {
+    const int d = I - a.fi0[f];
+    if (d < -3 || d > 3) continue;
+    if (KIND == INTERIOR && d == 0 && a.defer_i0 && J >= a.fdef[f][0] && J <= a.fdef[f][1] && K >= a.fdef[f][2] &&
+        K <= a.fdef[f][3])
+      return true;
+    if (__ldg(a.fflag[f] + J + (long)K * a.g.ny) & FL_SPLIT) return true;
+  }
+  return false;
+}
+
 #ifndef CGFD_PREFETCH
 #define CGFD_PREFETCH 1
 #endif
@@ -330,18 +410,18 @@ __device__ __forceinline__ bool locate_interior(const VolArgs &a, int &i, int &j
 #endif
 
 // resident blocks per SM asked of the compiler, per kernel kind (register
-// budget 65536 / (256 x blocks))
+// budget 65536 / (128 x blocks))
 #ifndef CGFD_LB_INTERIOR
-#define CGFD_LB_INTERIOR 4
+#define CGFD_LB_INTERIOR 8
 #endif
 #ifndef CGFD_LB_TOP
-#define CGFD_LB_TOP 3
+#define CGFD_LB_TOP 6
 #endif
 #ifndef CGFD_LB_SHELL
-#define CGFD_LB_SHELL 3
+#define CGFD_LB_SHELL 6
 #endif
 #ifndef CGFD_LB_FACE
-#define CGFD_LB_FACE 3
+#define CGFD_LB_FACE 6
 #endif
 
 template <int ID, int JD, int KD, int MODE, int KIND>
@@ -351,45 +431,27 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
     k_volume(const __grid_constant__ VolArgs a) {
   static_assert(KIND >= INTERIOR && KIND <= TOP, "kernel kind");
   const Grid &g = a.g;
+  const long sc = g.scmp;
   int i, j, k;
   if (KIND == INTERIOR ? !locate_interior(a, i, j, k) : !locate(a, i, j, k)) return;
   const int I = i + NG, J = j + NG, K = k + NG;
-  // split-node slabs (i0-3..i0+3 of unwelded nodes) belong to the fault
-  // kernels; with defer_i0 the fault planes go to the PLANE launch
-  for (int f = 0; f < a.nfault; f++) {
-    const int d = I - a.fi0[f];
-    if (KIND == INTERIOR && d == 0 && a.defer_i0 && J >= a.fdef[f][0] && J <= a.fdef[f][1] && K >= a.fdef[f][2] &&
-        K <= a.fdef[f][3])
-      return;
-    if (d >= -3 && d <= 3 && (__ldg(a.fflag[f] + J + (long)K * g.ny) & FL_SPLIT)) return;
-  }
   const long p = g.at(I, J, K);
-  const long sc = g.scmp;
+  if (other_kernels_point<KIND>(a, I, J, K)) return;
 #if CGFD_PREFETCH
-  if (MODE != RK_FIRST) {
-    // the RK update reads the time-n level (or, last, the V level) at its
-    // end: ask L2 for its lines now, so that those reads wait on L2, not DRAM
-    const real *l = MODE == RK_LAST ? a.end : a.pre;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(l + 4 * p));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(l + 4 * sc + 4 * p));
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(l + 8 * sc + p));
-  }
+  // the RK update reads the time-n level (in the last stage V) at its end:
+  // ask L2 for its lines now, so that those reads wait on L2, not DRAM
+  if (MODE != RK_FIRST) prefetch9(MODE == RK_LAST ? a.end : a.pre, sc, p);
 #if CGFD_AHEAD > 0
   if (KIND == INTERIOR) {
     // the DRAM misses of the block CGFD_AHEAD z rows up: the newest stencil
     // plane of the stage input and its coefficients (that block runs soon
     // after this one: blocks march up z within a y chunk)
-    const int kn = K + CGFD_AHEAD + (KD ? 3 : 1), kc = K + CGFD_AHEAD;
-    if (kn < g.nz) {
-      const long q = p + (long)(kn - K) * g.sz;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a.cur + 4 * q));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a.cur + 4 * sc + 4 * q));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a.cur + 8 * sc + q));
-    }
+    const int kc = K + CGFD_AHEAD, kn = kc + (KD ? 3 : 1);
+    if (kn < g.nz) prefetch9(a.cur, sc, p + (long)(kn - K) * g.sz);
     if (kc < g.nz) {
-      const long q = p + (long)CGFD_AHEAD * g.sz;
 #pragma unroll
-      for (int d = 0; d < 3; d++) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.coef + sc + 4 * (d * sc + q)));
+      for (int d = 0; d < 3; d++)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.coef + sc + 4 * (d * sc + p + (long)CGFD_AHEAD * g.sz)));
     }
   }
 #endif
@@ -403,8 +465,9 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
   }
 #endif
   const Taps w = taps_at(a.cur, sc, p);
+  const V9 c0 = tap9(w, 0);
   real v0[9];
-  ld9(w, 0, v0);
+  unpack9(c0, v0);
   const real4 r0 = coef_row(a.coef, sc, 0, p), r1 = coef_row(a.coef, sc, 1, p), r2 = coef_row(a.coef, sc, 2, p);
   const real e[3][3] = { { r0.x, r0.y, r0.z }, { r1.x, r1.y, r1.z }, { r2.x, r2.y, r2.z } };
   const real lam = r0.w, mu = r1.w, slw = r2.w;
@@ -416,18 +479,12 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
 
   real h[9];
   if (KIND == INTERIOR || KIND == PLANE) {
-    real G[3][3] = { { 0.f, 0.f, 0.f }, { 0.f, 0.f, 0.f }, { 0.f, 0.f, 0.f } };
+    real E[6] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
     real s[3] = { 0.f, 0.f, 0.f };
-    acc_dir<ID>(w, v0, ox, e[0], G, s);
-    acc_dir<JD>(w, v0, oy, e[1], G, s);
-    acc_dir<KD>(w, v0, oz, e[2], G, s);
-    h[VX] = slw * s[0]; h[VY] = slw * s[1]; h[VZ] = slw * s[2];
-    h[TXX] = l2m * G[0][0] + lam * (G[1][1] + G[2][2]);
-    h[TYY] = l2m * G[1][1] + lam * (G[0][0] + G[2][2]);
-    h[TZZ] = l2m * G[2][2] + lam * (G[0][0] + G[1][1]);
-    h[TXY] = mu * (G[0][1] + G[1][0]);
-    h[TXZ] = mu * (G[0][2] + G[2][0]);
-    h[TYZ] = mu * (G[1][2] + G[2][1]);
+    acc_dir<ID>(w, c0, ox, e[0], E, s);
+    acc_dir<JD>(w, c0, oy, e[1], E, s);
+    acc_dir<KD>(w, c0, oz, e[2], E, s);
+    rates(E, s, lam, mu, slw, h);
     rk_update<MODE>(a, p, v0, h);
     return;
   }
@@ -438,21 +495,17 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
     // auxiliary update
     constexpr int FD = KIND - FACE_X;
     constexpr int FF = FD == 0 ? ID : (FD == 1 ? JD : KD);
-    real G[3][3] = { { 0.f, 0.f, 0.f }, { 0.f, 0.f, 0.f }, { 0.f, 0.f, 0.f } };
+    real E[6] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
     real s[3] = { 0.f, 0.f, 0.f };
-    if (FD != 0) acc_dir<ID>(w, v0, ox, e[0], G, s);
-    if (FD != 1) acc_dir<JD>(w, v0, oy, e[1], G, s);
-    if (FD != 2) acc_dir<KD>(w, v0, oz, e[2], G, s);
+    if (FD != 0) acc_dir<ID>(w, c0, ox, e[0], E, s);
+    if (FD != 1) acc_dir<JD>(w, c0, oy, e[1], E, s);
+    if (FD != 2) acc_dir<KD>(w, c0, oz, e[2], E, s);
     real D[9], r[9], corr[9];
-    derivs<FF>(w, v0, FD == 0 ? ox : (FD == 1 ? oy : oz), D);
+    derivs<FF>(w, c0, FD == 0 ? ox : (FD == 1 ? oy : oz), D);
     rhs_dir(D, e[FD], lam, mu, l2m, slw, r);
-    h[VX] = slw * s[0] + r[VX]; h[VY] = slw * s[1] + r[VY]; h[VZ] = slw * s[2] + r[VZ];
-    h[TXX] = l2m * G[0][0] + lam * (G[1][1] + G[2][2]) + r[TXX];
-    h[TYY] = l2m * G[1][1] + lam * (G[0][0] + G[2][2]) + r[TYY];
-    h[TZZ] = l2m * G[2][2] + lam * (G[0][0] + G[1][1]) + r[TZZ];
-    h[TXY] = mu * (G[0][1] + G[1][0]) + r[TXY];
-    h[TXZ] = mu * (G[0][2] + G[2][0]) + r[TXZ];
-    h[TYZ] = mu * (G[1][2] + G[2][1]) + r[TYZ];
+    rates(E, s, lam, mu, slw, h);
+#pragma unroll
+    for (int c = 0; c < 9; c++) h[c] += r[c];
 #pragma unroll
     for (int c = 0; c < 9; c++) corr[c] = 0.f;
     if (a.pml[2 * FD].on) pml_face<MODE>(a, a.pml[2 * FD], FD, I, J, K, r, D, e[2], lam, mu, l2m, false, 0, corr);
@@ -473,7 +526,7 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
 #pragma unroll
   for (int c = 0; c < 9; c++) corr[c] = 0.f;
   // x
-  derivs<ID>(w, v0, ox, D);
+  derivs<ID>(w, c0, ox, D);
   dvx[0] = D[VX]; dvx[1] = D[VY]; dvx[2] = D[VZ];
   rhs_dir(D, e[0], lam, mu, l2m, slw, r);
 #pragma unroll
@@ -481,7 +534,7 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
   if (pml && a.pml[0].on) pml_face<MODE>(a, a.pml[0], 0, I, J, K, r, D, e[2], lam, mu, l2m, surfrow, fidx, corr);
   if (pml && a.pml[1].on) pml_face<MODE>(a, a.pml[1], 0, I, J, K, r, D, e[2], lam, mu, l2m, surfrow, fidx, corr);
   // y
-  derivs<JD>(w, v0, oy, D);
+  derivs<JD>(w, c0, oy, D);
   dvy[0] = D[VX]; dvy[1] = D[VY]; dvy[2] = D[VZ];
   rhs_dir(D, e[1], lam, mu, l2m, slw, r);
 #pragma unroll
@@ -489,7 +542,7 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
   if (pml && a.pml[2].on) pml_face<MODE>(a, a.pml[2], 1, I, J, K, r, D, e[2], lam, mu, l2m, surfrow, fidx, corr);
   if (pml && a.pml[3].on) pml_face<MODE>(a, a.pml[3], 1, I, J, K, r, D, e[2], lam, mu, l2m, surfrow, fidx, corr);
   // z
-  derivs<KD>(w, v0, oz, D);
+  derivs<KD>(w, c0, oz, D);
   rhs_dir(D, e[2], lam, mu, l2m, slw, r);
   if (pml && a.pml[4].on) pml_face<MODE>(a, a.pml[4], 2, I, J, K, r, D, e[2], lam, mu, l2m, false, fidx, corr);
   if (pml && a.pml[5].on) pml_face<MODE>(a, a.pml[5], 2, I, J, K, r, D, e[2], lam, mu, l2m, false, fidx, corr);

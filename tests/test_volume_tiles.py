@@ -1,0 +1,35 @@
+"""The volume kernels' tiles at the sizes where they change shape: interior
+boxes whose width leaves 0, 1, 8 (the most that join the x PML slab), 9 or
+31 columns beyond whole 32-point tiles, odd strike and depth sizes (a last
+block of each plane with one row at work), against the CPU oracle."""
+import numpy as np
+import pytest
+
+import inputs
+from cgfd import Solver, WAVE_COMPONENTS
+from oracle import OracleSolver
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("left", [0, 1, 8, 9, 31])
+def test_leftover_columns(cgfd_lib, oracle_built, left):
+    # 5-layer PML faces take 6 columns at either side; the fault's
+    # neighbourhood lies in the first tile
+    p = inputs.tpv_planar(ni=12 + 32 + left, nj=61, nk=37, fault_x_index=20, fault_grid=[15, 46, 12, 37], nuc_half=3,
+                          pml=5, nt=10, nsta=4, margin=10)
+    rng = np.random.default_rng(left)
+    g, o = Solver(p), OracleSolver(p)
+    wide = 32 if 0 < left <= 8 else 32 + left
+    rows = [61 - 12, 37 - 6 - 4]
+    assert wide * rows[0] * rows[1] - 7 * rows[0] * rows[1] < g.kernel_timing(1)[2] <= wide * rows[0] * rows[1]
+    for c in range(9):
+        f = (rng.standard_normal((p.nk, p.nj, p.ni)) * (1e-3 if c < 3 else 1e3)).astype(np.float32)
+        g.set_wavefield(c, f)
+        o.set_wavefield(c, f)
+    g.run(8)
+    o.run(8)
+    for c in range(9):
+        a, b = g.wavefield(c), o.wavefield(c)
+        # the float32 bound of the parity tests' random-state steps
+        assert np.linalg.norm(a - b) <= 2e-5 * np.linalg.norm(b), WAVE_COMPONENTS[c]
