@@ -21,8 +21,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 
 # (source, object, extra flags): the volume kernels build as one unit per
-# kernel kind so that they compile in parallel
-CU = [("volume.cu", f"volume_k{k}.cu.o", [f"-DCGFD_VOLUME_KIND={k}"]) for k in range(8)] + [
+# kernel kind, and per operator triple for those that hold every kind, so
+# that they compile in parallel
+CU = [("volume.cu", f"volume_k{k}.cu.o", [f"-DCGFD_VOLUME_KIND={k}"]) for k in range(16)] + [
     (f, f + ".o", []) for f in ("fault.cu", "boundary.cu", "noalloc.cu", "api.cu")]
 CPP = ["setup.cpp"]
 DRIVER = os.path.join(HERE, "driver")

@@ -25,7 +25,8 @@
 #include "setup.h"
 
 namespace cgfd {
-void volume_boxes(VolArgs &a, const int (*boxes)[6], int n, bool pack);
+bool volume_boxes(VolArgs &a, int kind, const int (*boxes)[6], int n, bool pack);
+void launch_volume_all(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st);
 void launch_volume_interior(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st);
 void launch_volume_shell(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st);
 void launch_volume_face_x(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st);
@@ -34,7 +35,7 @@ void launch_volume_face_z(const VolArgs &a, int idir, int jdir, int kdir, int mo
 void launch_volume_edge(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st);
 void launch_volume_plane(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st);
 void launch_volume_top(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st);
-int launch_fault_pre(const FaultArgs &a, cudaStream_t st);
+int launch_fault_pre(const FaultArgs &a, const StationArgs *rec, cudaStream_t st);
 int launch_fault_post(const FaultArgs &a, cudaStream_t st);
 cudaError_t noalloc_scratch_address(real **p);
 void launch_record(const StationArgs &a, cudaStream_t st);
@@ -122,6 +123,8 @@ struct cgfd_solver {
   // interior kernel (CGFD_POST_EARLY)
   bool post_early = true;
   cudaEvent_t ev_stage[4] = {}, ev_predone[4] = {}, ev_postdone[4] = {};
+  // the boundary kinds in one launch (small grids; CGFD_MERGED)
+  bool merged = false;
   double run_ms = 0, vol_ms = 0, int_ms = 0;
   long long vol_launches = 0, int_launches = 0;
   long long int_points = 0, vol_points = 0;   // points one launch updates
@@ -289,6 +292,46 @@ void fault_planes(const cgfd_solver *s, VolArgs &v) {
   }
 }
 
+// Grids up to this many points launch their boundary kinds together: small
+// ones are bound by the chain of dependent launches and by launches that do
+// not fill the GPU, large ones by bytes, where each kind's own code and
+// register count pay.  Without a free surface there are two kinds fewer to
+// chain.  Measured, step apart / together: free surface 0.06 M points
+// 167 / 102 us, 0.24 M (no fault) 193 / 93, 0.46 M 320 / 241, 0.91 M 399 / 329,
+// 1.28 M 453 / 403, 1.94 M 564 / 505, 3.39 M 804 / 800, 5.24 M 1157 / 1159;
+// PML on all faces 0.06 M 119 / 95, 0.14 M 145 / 119, 0.27 M 167 / 157,
+// 0.39 M 201 / 203, 1.28 M 391 / 406, without a fault 0.91 M 254 / 229.
+long long merge_points(const cgfd_solver *s) {
+  return s->isfree ? 3'500'000 : (s->faults.empty() ? 1'000'000 : 300'000);
+}
+
+// the boundary boxes of a small grid's one boundary launch, the kinds with
+// the longest points first; the surface rows with `top`
+bool merged_boxes(const cgfd_solver *s, VolArgs &v, bool top) {
+  bool ok = true;
+  if (top) ok &= volume_boxes(v, 7, s->kbox[7], s->nkbox[7], s->pack);
+  for (int kind : { 1, 5, 2, 3, 4 }) ok &= volume_boxes(v, kind, s->kbox[kind], s->nkbox[kind], s->pack);
+  return ok;
+}
+// the boxes of the launch after the split nodes: the surface rows, and the
+// fault planes that the earlier launches deferred, each in the kind of the
+// box it lies in
+bool late_boxes(const cgfd_solver *s, VolArgs &v) {
+  bool ok = volume_boxes(v, 7, s->kbox[7], s->nkbox[7], s->pack);
+  for (auto &F : s->faults) {
+    if (F.nj <= 0 || F.nk <= 0) continue;
+    const int r[6] = { F.d.i0 - NG, F.d.i0 - NG, F.j0 - 3, F.j0 + F.nj + 2, F.k0 - 3, F.k0 + F.nk + 2 };
+    for (int kind = 0; kind < 6; kind++)
+      for (int b = 0; b < s->nkbox[kind]; b++) {
+        const int *B = s->kbox[kind][b];
+        const int cut[1][6] = { { std::max(B[0], r[0]), std::min(B[1], r[1]), std::max(B[2], r[2]), std::min(B[3], r[3]),
+                                  std::max(B[4], r[4]), std::min(B[5], r[5]) } };
+        ok &= volume_boxes(v, kind, cut, 1, true);
+      }
+  }
+  return ok;
+}
+
 void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = true) {
   const int ip = it % 8;
   const bool tm = s->timing && timed;
@@ -296,7 +339,13 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
   StationArgs sa{};
   sa.g = s->g; sa.st = s->st; sa.w = s->w[slot(LP, it)]; sa.ns = (long)s->g.ny * s->g.nz; sa.ctl = s->ctl;
   for (size_t f = 0; f < s->faults.size(); f++) sa.fout[f] = s->faults[f].out;
-  if ((s->st.n + s->st.nf) > 0 && s->st.max_rec > 0) { launch_record(sa, s->stream); nl++; }
+  // the stations are sampled before the step changes anything: with a fault
+  // in its first kernel of the first stage, else in a launch of their own
+  const bool rec = (s->st.n + s->st.nf) > 0 && s->st.max_rec > 0;
+  if (rec && s->faults.empty()) { launch_record(sa, s->stream); nl++; }
+  auto fault_pre = [&](int stage, const FaultArgs *fa, int n, cudaStream_t st) {
+    for (int f = 0; f < n; f++) nl += launch_fault_pre(fa[f], rec && stage == 0 && f == 0 ? &sa : nullptr, st);
+  };
   // the fault kernels' arguments of one stage
   auto stage_fargs = [&](int stage, FaultArgs *fa) {
     const int idir = (kPairs[ip][0] + stage) % 2, jdir = (kPairs[ip][1] + stage) % 2, kdir = (kPairs[ip][2] + stage) % 2;
@@ -353,14 +402,87 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
   const bool pe2 = ov && s->post_early;
   FaultArgs fargs[MAXF], fnext[MAXF];
   const int nfa = stage_fargs(0, fargs);
-  for (int stage = 0; stage < 4; stage++) {
-    const int idir = (kPairs[ip][0] + stage) % 2, jdir = (kPairs[ip][1] + stage) % 2, kdir = (kPairs[ip][2] + stage) % 2;
-    const int mode = stage;   // RK_FIRST .. RK_LAST
+  // small grids (merge_points): one launch of all PML kinds and one of the
+  // interior box side by side with the fault kernels, then one of the surface
+  // rows and the fault planes beside the fault slabs.  The timed graphs keep
+  // the separate kernels' schedule, in which the interior launch is timed
+  const bool merged = s->merged && !tm;
+  // the volume kernels' arguments of one stage, without boxes
+  auto stage_vargs = [&](int stage) {
     const int Lcur = stage == 0 ? LP : (stage == 2 ? LB : LA);
     const int Lout = stage == 0 ? LA : (stage == 1 ? LB : (stage == 2 ? LA : -1));
-    const real ca = stage < 3 ? kRkA[stage] * s->dt : RL(0.0), cb = kRkB[stage] * s->dt;
     const int scur = slot(Lcur, it), spre = slot(LP, it), send = slot(LE, it);
     const int sout = Lout >= 0 ? slot(Lout, it) : -1;
+    VolArgs v{};
+    v.g = s->g; v.cur = s->w[scur]; v.pre = s->w[spre]; v.out = sout >= 0 ? s->w[sout] : nullptr; v.end = s->w[send];
+    v.coef = s->coef; v.free_mat = s->free_mat;
+    v.ca = stage < 3 ? kRkA[stage] * s->dt : RL(0.0); v.cb = kRkB[stage] * s->dt; v.isfree = s->isfree;
+    v.nfault = (int)s->faults.size();
+    fault_planes(s, v);
+    for (int q = 0; q < 6; q++) {
+      v.pml[q] = s->pml[q].d;
+      if (!v.pml[q].on) continue;
+      v.pml[q].acur = s->pml[q].aux[scur]; v.pml[q].apre = s->pml[q].aux[spre];
+      v.pml[q].aout = sout >= 0 ? s->pml[q].aux[sout] : nullptr; v.pml[q].aend = s->pml[q].aux[send];
+    }
+    return v;
+  };
+  auto merged_stage = [&](int stage) {
+    const int idir = (kPairs[ip][0] + stage) % 2, jdir = (kPairs[ip][1] + stage) % 2, kdir = (kPairs[ip][2] + stage) % 2;
+    VolArgs v = stage_vargs(stage);
+    // with the surface rows in the shell kind (CGFD_TOP=0) nothing is
+    // deferred and the volume launch waits for the split nodes
+    const bool defer = nfa > 0 && (!s->isfree || s->nkbox[7] > 0);
+    if (nfa > 0) {
+      if (stage > 0) stage_fargs(stage, fargs);
+      cudaEventRecord(s->ev_stage[stage], s->stream);
+      cudaStreamWaitEvent(s->aux[0], s->ev_stage[stage], 0);
+      fault_pre(stage, fargs, nfa, s->aux[0]);
+      cudaEventRecord(s->ev_predone[stage], s->aux[0]);
+      for (int f = 0; f < nfa; f++) nl += launch_fault_post(fargs[f], s->aux[0]);
+      cudaEventRecord(s->ev_postdone[stage], s->aux[0]);
+      if (!defer) cudaStreamWaitEvent(s->stream, s->ev_predone[stage], 0);
+    }
+    VolArgs vi = v;
+    vi.defer_i0 = defer ? 1 : 0;
+    VolArgs vb = vi;
+    merged_boxes(s, vb, !defer);
+    if (vb.nbox > 0) {
+      // first, on its own stream: its points take longest
+      cudaEventRecord(s->ev_fork[stage], s->stream);
+      cudaStreamWaitEvent(s->aux[2], s->ev_fork[stage], 0);
+      launch_volume_all(vb, idir, jdir, kdir, stage, s->aux[2]);
+      nl++;
+    }
+    volume_boxes(vi, 0, s->kbox[0], s->nkbox[0], false);
+    vi.ychunk = s->ychunk;
+    if (vi.nbox > 0) {
+      launch_volume_interior(vi, idir, jdir, kdir, stage, s->stream);
+      nl++;
+    }
+    if (vb.nbox > 0) {
+      cudaEventRecord(s->ev_join[stage][2], s->aux[2]);
+      cudaStreamWaitEvent(s->stream, s->ev_join[stage][2], 0);
+    }
+    if (defer) {
+      late_boxes(s, v);
+      if (v.nbox > 0) {
+        cudaStreamWaitEvent(s->aux[1], s->ev_predone[stage], 0);
+        launch_volume_all(v, idir, jdir, kdir, stage, s->aux[1]);
+        nl++;
+        cudaEventRecord(s->ev_join[stage][1], s->aux[1]);
+        cudaStreamWaitEvent(s->stream, s->ev_join[stage][1], 0);
+      }
+    }
+    if (nfa > 0) cudaStreamWaitEvent(s->stream, s->ev_postdone[stage], 0);
+  };
+  for (int stage = 0; stage < 4; stage++) {
+    if (merged) {
+      merged_stage(stage);
+      continue;
+    }
+    const int idir = (kPairs[ip][0] + stage) % 2, jdir = (kPairs[ip][1] + stage) % 2, kdir = (kPairs[ip][2] + stage) % 2;
+    const int mode = stage;   // RK_FIRST .. RK_LAST
     if (stage > 0) {
       if (early) std::memcpy(fargs, fnext, sizeof(FaultArgs) * nfa);
       else stage_fargs(stage, fargs);
@@ -371,14 +493,14 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
         // fault planes), once the stage input is complete
         cudaEventRecord(s->ev_stage[stage], s->stream);
         cudaStreamWaitEvent(s->aux[0], s->ev_stage[stage], 0);
-        for (int f = 0; f < nfa; f++) nl += launch_fault_pre(fargs[f], s->aux[0]);
+        fault_pre(stage, fargs, nfa, s->aux[0]);
         cudaEventRecord(s->ev_predone[stage], s->aux[0]);
         if (pe2) {
           for (int f = 0; f < nfa; f++) nl += launch_fault_post(fargs[f], s->aux[0]);
           cudaEventRecord(s->ev_postdone[stage], s->aux[0]);
         }
       } else {
-        for (int f = 0; f < nfa; f++) nl += launch_fault_pre(fargs[f], s->stream);
+        fault_pre(stage, fargs, nfa, s->stream);
       }
     }
     // external event nodes when captured, so that the events really fire
@@ -394,20 +516,8 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
     }
     if (!br2)
       for (int f = 0; f < nfa; f++) nl += launch_fault_post(fargs[f], st_fault);
-    VolArgs v{};
-    v.g = s->g; v.cur = s->w[scur]; v.pre = s->w[spre]; v.out = sout >= 0 ? s->w[sout] : nullptr; v.end = s->w[send];
-    v.coef = s->coef; v.free_mat = s->free_mat;
-    v.ca = ca; v.cb = cb; v.isfree = s->isfree;
-    v.nfault = (int)s->faults.size();
-    v.defer_i0 = ov ? 1 : 0;
-    fault_planes(s, v);
-    for (int q = 0; q < 6; q++) {
-      v.pml[q] = s->pml[q].d;
-      if (!v.pml[q].on) continue;
-      v.pml[q].acur = s->pml[q].aux[scur]; v.pml[q].apre = s->pml[q].aux[spre];
-      v.pml[q].aout = sout >= 0 ? s->pml[q].aux[sout] : nullptr; v.pml[q].aend = s->pml[q].aux[send];
-    }
-    VolArgs vs = v;
+    VolArgs vs = stage_vargs(stage);
+    vs.defer_i0 = ov ? 1 : 0;
     {
       // interior box, single-direction PML slabs, generic shell
       const int kind0 = 0;
@@ -417,7 +527,8 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
           // (which refresh the split nodes there) are done
           cudaStreamWaitEvent(s->stream, s->ev_predone[stage], 0);
           VolArgs vp = vs;
-          volume_boxes(vp, s->kbox[6], s->nkbox[6], true);
+          vp.defer_i0 = 0;
+          volume_boxes(vp, 6, s->kbox[6], s->nkbox[6], true);
           if (vp.nbox > 0) { launch_volume_plane(vp, idir, jdir, kdir, mode, s->stream); nl++; }
         }
         if (kind == 1 && br2) {
@@ -438,7 +549,7 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
           cudaEventRecord(s->ev_pre[stage], s->stream);
           cudaStreamWaitEvent(st_fault, s->ev_pre[stage], 0);
           stage_fargs(stage + 1, fnext);
-          for (int f = 0; f < nfa; f++) nl += launch_fault_pre(fnext[f], st_fault);
+          fault_pre(stage + 1, fnext, nfa, st_fault);
           if (ov) cudaEventRecord(s->ev_predone[stage + 1], st_fault);
           if (pe2) {
             // the slab points' input is complete as well (the PML boxes
@@ -453,11 +564,13 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
           // surface rows away from every PML face, beside (before) the
           // shell's rows in the PML columns
           VolArgs vt = vs;
-          volume_boxes(vt, s->kbox[7], s->nkbox[7], s->pack);
+          vt.defer_i0 = 0;
+          volume_boxes(vt, 7, s->kbox[7], s->nkbox[7], s->pack);
           if (vt.nbox > 0) { launch_volume_top(vt, idir, jdir, kdir, mode, st_pml); nl++; }
         }
         VolArgs vk = vs;
-        volume_boxes(vk, s->kbox[kind], s->nkbox[kind], kind != 0 && s->pack);
+        if (kind != 0) vk.defer_i0 = 0;
+        volume_boxes(vk, kind, s->kbox[kind], s->nkbox[kind], kind != 0 && s->pack);
         vk.ychunk = s->ychunk;
         if (vk.nbox == 0) continue;
         switch (kind) {
@@ -507,11 +620,12 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
   if (s->isfree) {
     PeakArgs pa{};
     pa.g = s->g; pa.wend = s->w[slot(LE, it)]; pa.wpre = s->w[slot(LP, it)];
-    pa.pg = s->pg; pa.dis = s->dis; pa.dt = s->dt;
+    pa.pg = s->pg; pa.dis = s->dis; pa.dt = s->dt; pa.ctl = s->ctl; pa.max_rec = s->st.max_rec;
     nl += launch_surface_peaks(pa, s->stream);
+  } else {
+    launch_advance(s->ctl, s->st.max_rec, s->stream);
+    nl++;
   }
-  launch_advance(s->ctl, s->st.max_rec, s->stream);
-  nl++;
   s->launches_per_step = nl;
 }
 
@@ -660,7 +774,7 @@ static cudaError_t tune_ychunk(cgfd_solver *s) {
   v.ca = kRkA[0] * s->dt; v.cb = kRkB[0] * s->dt; v.isfree = s->isfree;
   v.nfault = (int)s->faults.size();
   fault_planes(s, v);
-  volume_boxes(v, s->kbox[0], s->nkbox[0], false);
+  volume_boxes(v, 0, s->kbox[0], s->nkbox[0], false);
   cudaEvent_t t0, t1;
   if ((e = cudaEventCreate(&t0)) != cudaSuccess) return e;
   if ((e = cudaEventCreate(&t1)) != cudaSuccess) { cudaEventDestroy(t0); return e; }
@@ -905,6 +1019,16 @@ int cgfd_upload(const cgfd_setup *su, cgfd_solver **out) {
     if (po && po[0] == '0') s->pre_overlap = false;
     const char *pq = std::getenv("CGFD_POST_EARLY");
     if (pq && pq[0] == '0') s->post_early = false;
+    {
+      VolArgs m{}, l{};
+      const bool fits = merged_boxes(s, m, true) && late_boxes(s, l);
+      s->merged = m.nbox > 0 && (long long)ni * nj * nk <= merge_points(s);
+      for (const char *e : { "CGFD_BRANCHES", "CGFD_PRE_OVERLAP", "CGFD_POST_EARLY", "CGFD_PRE_EARLY" })
+        if (std::getenv(e)) s->merged = false;    // switches of the separate kernels' schedule
+      const char *me = std::getenv("CGFD_MERGED");
+      if (me) s->merged = me[0] != '0';
+      if (!fits) s->merged = false;
+    }
     const char *pk = std::getenv("CGFD_PACK");
     if (pk && pk[0] == '0') s->pack = false;
     // y tiles (kTileY rows) per interior chunk: the z window of a chunk, about 8
@@ -1319,12 +1443,17 @@ int cgfd_ensemble_run(cgfd_ensemble *e, int nsteps) {
         // its interior kernel (measured: +2% over the solo default); the
         // schedules change no arithmetic
         const int br0 = s->branches;
-        const bool pe0 = s->post_early;
+        const bool pe0 = s->post_early, me0 = s->merged;
         if (s->branches == 3) s->branches = 2;
         s->post_early = false;
+        // nor do its boundary kinds share a launch: other members fill the
+        // GPU (16 members of 0.12 M points 946 against 1003 us per step, 12
+        // of 0.69 M 2719 against 2982)
+        s->merged = false;
         enqueue_step(s, it, nullptr, false);
         s->branches = br0;
         s->post_early = pe0;
+        s->merged = me0;
         cudaEventRecord(e->join[q], s->stream);
         cudaStreamWaitEvent(e->origin, e->join[q], 0);
       }

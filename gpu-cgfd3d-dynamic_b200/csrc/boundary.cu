@@ -43,6 +43,11 @@ __global__ void __launch_bounds__(256) k_sponge(const SpongeArgs a) {
 __global__ void __launch_bounds__(256) k_surface_peaks(const PeakArgs a) {
   const Grid &g = a.g;
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (i == 0 && j == 0) {
+    // the step ends here: count it (and its station record)
+    a.ctl->it += 1;
+    if (a.ctl->nrec < a.max_rec) a.ctl->nrec += 1;
+  }
   if (i >= g.ni || j >= g.nj) return;
   const long p = g.at(i + NG, j + NG, g.nk + NG - 1);
   // velocities are the first three lanes of the first 16-byte group
@@ -63,11 +68,14 @@ __global__ void __launch_bounds__(256) k_surface_peaks(const PeakArgs a) {
       fabs(v1.x), fabs(v1.y), fabs(v1.z),
       sqrt(Ax * Ax + Ay * Ay + Az * Az), sqrt(Ax * Ax + Ay * Ay), Ax, Ay, Az,
       sqrt(Dx * Dx + Dy * Dy + Dz * Dz), sqrt(Dx * Dx + Dy * Dy), fabs(Dx), fabs(Dy), fabs(Dz) };
+  // all peaks are read before the first is written: the compiler cannot tell
+  // them apart, and 15 dependent round trips made the launch 11 us long
+  real old[15];
 #pragma unroll
-  for (int c = 0; c < 15; c++) {
-    real *o = a.pg + c * n + q;
-    if (*o < val[c]) *o = val[c];
-  }
+  for (int c = 0; c < 15; c++) old[c] = a.pg[c * n + q];
+#pragma unroll
+  for (int c = 0; c < 15; c++)
+    if (old[c] < val[c]) a.pg[c * n + q] = val[c];
 }
 
 }  // namespace

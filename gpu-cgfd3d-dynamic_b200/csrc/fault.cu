@@ -4,15 +4,15 @@
 // traction + slip-weakening friction kernel, fault2wave, the fault velocity
 // RHS, the fault stress RHS (forward or backward variant), two fault RK
 // updates, fault2wave again and the stage traction update, each as its own
-// kernel (src/forward/drv_rk_curv_col.cu:277-588).  Here that becomes four
+// kernel (src/forward/drv_rk_curv_col.cu:277-588).  Here that becomes three
 // kernels over the fault plane:
 //
-//   k_fault_weld    welded nodes: fault wavefield from the volume at i0
-//                   (wave2fault_gpu, src/forward/transform.cu:101-212)
-//   k_fault_trac    tractions J e . sigma of the stage input at the volume
+//   k_fault_pre     welded nodes: fault wavefield from the volume at i0
+//                   (wave2fault_gpu, src/forward/transform.cu:101-212);
+//                   tractions J e . sigma of the stage input at the volume
 //                   points i0-6..i0+6 around the split box, once each, into a
 //                   per-fault scratch array read by the next two kernels
-//   k_fault_split   split nodes, one thread each, in one pass:
+//   k_fault_split   split nodes, six threads each, in one pass:
 //                   T1 traction image, trial traction and linear
 //                   slip-weakening friction (trial_slipweakening_gpu,
 //                   src/forward/trial_slipweakening.cu:92-388), stage
@@ -77,32 +77,19 @@ __device__ __forceinline__ void odd_image(real v[7], int nf) {
   }
 }
 
-// RK stage update of N values (see RK_FIRST in ops.cuh); every level read
-// is issued before the first store (the compiler cannot prove that the
-// levels do not alias, and interleaved load / store pairs cost one memory
-// round trip each)
-template <int N>
-__device__ __forceinline__ void rk_put_n(int mode, real ca, real cb, const real *cur, const real *pre,
-                                         real *out, real *end, const long o[N], const real h[N]) {
-  real u[N], e[N];
-#pragma unroll
-  for (int n = 0; n < N; n++) {
-    if (mode != RK_THIRD) u[n] = cur[o[n]];
-    if (mode != RK_FIRST) e[n] = mode == RK_LAST ? end[o[n]] : pre[o[n]];
+// RK stage update (see RK_FIRST in ops.cuh) of one value: u0 the time-n
+// level's (in the last stage V), cur the stage input's, h its rate; returns
+// the value written to the next stage's input (in the last stage time n+1)
+__device__ __forceinline__ real rk_put(int mode, real ca, real cb, real u0, real cur, real h, real *out, real *end) {
+  if (mode == RK_LAST) {
+    const real r = rk_end(u0, cur, cb * h);
+    *end = r;
+    return r;
   }
-  if (mode == RK_FIRST) {
-#pragma unroll
-    for (int n = 0; n < N; n++) out[o[n]] = rk_out(u[n], ca * h[n]);
-  } else if (mode == RK_LAST) {
-#pragma unroll
-    for (int n = 0; n < N; n++) end[o[n]] = rk_end(e[n], u[n], cb * h[n]);
-  } else {
-#pragma unroll
-    for (int n = 0; n < N; n++) {
-      out[o[n]] = rk_out(e[n], ca * h[n]);
-      if (mode == RK_SECOND) end[o[n]] = rk_v(e[n], u[n], ca * h[n]);
-    }
-  }
+  const real r = rk_out(mode == RK_FIRST ? cur : u0, ca * h);
+  *out = r;
+  if (mode == RK_SECOND) *end = rk_v(u0, cur, ca * h);
+  return r;
 }
 
 // slot of x offset d (-6..-1, 1..6) in the traction scratch
@@ -111,8 +98,12 @@ __device__ __forceinline__ int trac_slot(int d) { return d < 0 ? d + 6 : d + 5; 
 // split-node volume point from the fault fields (fault2wave_gpu,
 // transform.cu:293-376): velocity = mean of the two sides, stress from the
 // traction vectors [T1 | mean T2 | mean T3] through the inverse metric.
-__device__ void split_to_volume(const Grid &g, const real *__restrict__ cf, long sc, long ns, long nd,
-                                int i0, int J, int K, const real *f, const real T1[3], real *wt) {
+// V, T2, T3: the node's values of one component and side, [3 side + component]
+// entries `st` apart.
+__device__ __forceinline__ void split_to_volume(const Grid &g, const real *__restrict__ cf, int i0, int J, int K,
+                                                const real *V, const real *T2, const real *T3, int st, const real T1[3],
+                                                real *wt) {
+  const long sc = g.scmp;
   const long p0 = g.at(i0, J, K);
   real mt[3][3];   // columns e_xi, e_eta, e_zeta
 #pragma unroll
@@ -125,8 +116,8 @@ __device__ void split_to_volume(const Grid &g, const real *__restrict__ cf, long
 #pragma unroll
   for (int r = 0; r < 3; r++) {
     tr[r][0] = T1[r];
-    tr[r][1] = (f[fidx(FT2X + r, 0, ns, nd)] + f[fidx(FT2X + r, 1, ns, nd)]) * 0.5f;
-    tr[r][2] = (f[fidx(FT3X + r, 0, ns, nd)] + f[fidx(FT3X + r, 1, ns, nd)]) * 0.5f;
+    tr[r][1] = (T2[r * st] + T2[(3 + r) * st]) * 0.5f;
+    tr[r][2] = (T3[r * st] + T3[(3 + r) * st]) * 0.5f;
   }
   const real c00 = mt[1][1] * mt[2][2] - mt[2][1] * mt[1][2], c01 = mt[2][1] * mt[0][2] - mt[0][1] * mt[2][2];
   const real c02 = mt[0][1] * mt[1][2] - mt[0][2] * mt[1][1], c10 = mt[1][2] * mt[2][0] - mt[1][0] * mt[2][2];
@@ -135,30 +126,30 @@ __device__ void split_to_volume(const Grid &g, const real *__restrict__ cf, long
   const real c22 = mt[0][0] * mt[1][1] - mt[0][1] * mt[1][0];
   const real id = 1.0f / (c00 * mt[0][0] + c01 * mt[1][0] + c02 * mt[2][0]);
   const real mi[3][3] = { { c00 * id, c01 * id, c02 * id }, { c10 * id, c11 * id, c12 * id }, { c20 * id, c21 * id, c22 * id } };
-  real st[3][3];
+  real sg[3][3];
 #pragma unroll
   for (int r = 0; r < 3; r++)
 #pragma unroll
-    for (int c = 0; c < 3; c++) st[r][c] = (tr[r][0] * mi[0][c] + tr[r][1] * mi[1][c] + tr[r][2] * mi[2][c]) * rj;
+    for (int c = 0; c < 3; c++) sg[r][c] = (tr[r][0] * mi[0][c] + tr[r][1] * mi[1][c] + tr[r][2] * mi[2][c]) * rj;
   real u[3];
 #pragma unroll
-  for (int c = 0; c < 3; c++) u[c] = (f[fidx(FVX + c, 0, ns, nd)] + f[fidx(FVX + c, 1, ns, nd)]) * 0.5f;
-  reinterpret_cast<real4 *>(wt)[p0] = make_real4(u[0], u[1], u[2], st[0][0]);
+  for (int c = 0; c < 3; c++) u[c] = (V[c * st] + V[(3 + c) * st]) * 0.5f;
+  reinterpret_cast<real4 *>(wt)[p0] = make_real4(u[0], u[1], u[2], sg[0][0]);
   // the reference's fault2wave_gpu receives Tyz and Txz in swapped
   // positions (transform.cu:281-289 vs :293-300); kept for parity
   reinterpret_cast<real4 *>(wt + 4 * sc)[p0] =
-      make_real4(st[1][1], st[2][2], (st[0][2] + st[2][0]) * 0.5f, (st[1][2] + st[2][1]) * 0.5f);
-  wt[g.w(TXY, p0)] = (st[0][1] + st[1][0]) * 0.5f;
+      make_real4(sg[1][1], sg[2][2], (sg[0][2] + sg[2][0]) * 0.5f, (sg[1][2] + sg[2][1]) * 0.5f);
+  wt[g.w(TXY, p0)] = (sg[0][1] + sg[1][0]) * 0.5f;
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
-__global__ void k_fault_weld(const FaultArgs a) {
+// welded node t of the box wj0.., wk0..
+__device__ __forceinline__ void weld_node(const FaultArgs &a, long t) {
   const Grid &g = a.g;
-  const int j = a.wj0 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = a.wk0 + blockIdx.y * blockDim.y + threadIdx.y;
-  if (j >= a.wj0 + a.wnj || k >= a.wk0 + a.wnk) return;
+  if (t >= (long)a.wnj * a.wnk) return;
+  const int k = a.wk0 + (int)(t / a.wnj), j = a.wj0 + (int)(t % a.wnj);
   const int J = j + NG, K = k + NG;
   const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny;
   if (a.F.flag[nd] & FL_SPLIT) return;
@@ -186,9 +177,8 @@ __global__ void k_fault_weld(const FaultArgs a) {
 // T3 = J e_zeta . sigma at x = i0+-1..3.  The trial, friction and slab
 // velocity kernels read them from here instead of recomputing each one
 // (10 loads) for every tap.  Layout [9][tnk][tnj][12], x offset fastest.
-__global__ void __launch_bounds__(192) k_fault_trac(const FaultArgs a) {
+__device__ __forceinline__ void trac_item(const FaultArgs &a, long t) {
   const Grid &g = a.g;
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const long node = t / 12;
   if (node >= (long)a.tnj * a.tnk) return;
   const int slot = (int)(t - node * 12);
@@ -206,138 +196,6 @@ __global__ void __launch_bounds__(192) k_fault_trac(const FaultArgs a) {
     trac3(g, a.wcur, a.coef, q, 2, v);
     tp[6 * pl] = v[0]; tp[7 * pl] = v[1]; tp[8 * pl] = v[2];
   }
-}
-
-// ---------------------------------------------------------------------------
-// split nodes, one thread per node: trial traction and linear slip-weakening
-// friction (trial_slipweakening_gpu), the stage traction output, the refresh
-// of the stage input's split-node volume point, and the split-node velocity
-// RHS with its RK update
-__device__ __forceinline__ void split_trial(const FaultArgs &a, int j, int k, uint8_t fl) {
-  const Grid &g = a.g;
-  const int J = j + NG, K = k + NG;
-  const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny, sc = g.scmp;
-  const FaultDev &F = a.F;
-  const int i0 = F.i0;
-  const real *cf = a.coef;
-  const long ny = g.ny;
-  const int km = g.nk - (k + 1);
-  const bool surf = a.isfree && km <= 3;
-  const int nf = km + 3;
-
-  // T1 = J e_xi . sigma at i0-3..i0+3 (index 3 is the split node, filled
-  // after the friction law)
-  real X1[7][3];
-  const long pl = (long)a.tnj * a.tnk * 12;
-  const real *tr = a.trac + ((long)(K - a.tk0) * a.tnj + (J - a.tj0)) * 12;
-#pragma unroll
-  for (int l = -3; l <= 3; l++) {
-    if (l == 0) continue;
-#pragma unroll
-    for (int c = 0; c < 3; c++) X1[l + 3][c] = tr[c * pl + trac_slot(l)];
-  }
-
-  // along-fault derivatives of the fault tractions, both sides
-  real DyT2[2][3], DzT3[2][3], R[2][3];
-#pragma unroll
-  for (int m = 0; m < 2; m++) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const real *t2 = a.fc + fidx(FT2X + c, m, ns, nd);
-      DyT2[m][c] = (fl & FL_RUPY) ? mac22(t2, 1, a.jdir) : drp_rt(t2, 1, a.jdir);
-      const real *t3 = a.fc + fidx(FT3X + c, m, ns, nd);
-      real dz;
-      if (surf) {
-        // traction image of T3 about the free surface
-        real v[7];
-#pragma unroll
-        for (int l = 0; l < 7; l++) v[l] = __ldg(t3 + (long)(l - 3) * ny);
-        odd_image(v, nf);
-        dz = drp_v(v + 3, a.kdir);
-      } else {
-        dz = (fl & FL_RUPZ) ? mac22(t3, ny, a.kdir) : drp_rt(t3, ny, a.kdir);
-      }
-      DzT3[m][c] = dz;
-      const int s = 2 * m - 1;
-      const real img = kA1 * X1[3 + s][c] + kA2 * X1[3 + 2 * s][c] + kA3 * X1[3 + 3 * s][c];
-      R[m][c] = 0.5f * ((real)s * img + (DyT2[m][c] + DzT3[m][c]));
-    }
-  }
-
-  // trial traction from the velocity jump of time level n and friction
-  const long p0 = g.at(i0, J, K);
-  const real jac0 = coef_jac(cf, p0);
-  const real rho0 = F.scal[FS_RHO0 * ns + nd], rho1 = F.scal[FS_RHO1 * ns + nd];
-  const real M0 = 0.5f * jac0 * rho0, M1 = 0.5f * jac0 * rho1;
-  real Tr[3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const real dV = a.fp[fidx(FVX + c, 1, ns, nd)] - a.fp[fidx(FVX + c, 0, ns, nd)];
-    Tr[c] = 2.0f * (M0 * M1 * dV / a.dt + M0 * R[1][c] - M1 * R[0][c]) / (kA0 * (M0 + M1));
-  }
-  const real4 exi = coef_row(cf, sc, 0, p0);
-  real vn[3] = { exi.x, exi.y, exi.z };
-  const real vn0 = sqrt(vn[0] * vn[0] + vn[1] * vn[1] + vn[2] * vn[2]);
-  const real jacvec = jac0 * vn0;
-  vn[0] /= vn0; vn[1] /= vn0; vn[2] /= vn0;
-  const real T0[3] = { F.scal[FS_T0X * ns + nd], F.scal[FS_T0Y * ns + nd], F.scal[FS_T0Z * ns + nd] };
-  real Tl[3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) Tl[c] = Tr[c] / jacvec + T0[c];
-  const real Tn0 = Tl[0] * vn[0] + Tl[1] * vn[1] + Tl[2] * vn[2];
-  real Ts[3] = { Tl[0] - vn[0] * Tn0, Tl[1] - vn[1] * Tn0, Tl[2] - vn[2] * Tn0 };
-  const real Ts0 = sqrt(Ts[0] * Ts[0] + Ts[1] * Ts[1] + Ts[2] * Ts[2]);
-  bool change = false;
-  real Tau_n = Tn0;
-  if (Tn0 >= 0.f) { Tau_n = 0.f; change = true; }     // the fault cannot open
-  const real slip = F.out[CGFD_FAULT_SLIP * ns + nd];
-  const real mus = F.scal[FS_MUS * ns + nd], mud = F.scal[FS_MUD * ns + nd];
-  const real Dc = F.scal[FS_DC * ns + nd], C0 = F.scal[FS_C0 * ns + nd];
-  const real fr = slip <= Dc ? mus - (mus - mud) * slip / Dc : mud;
-  const real Tau_c = -fr * Tau_n + C0;
-  real Tau_s = Ts0;
-  if (Ts0 >= Tau_c) { Tau_s = Tau_c; change = true; }
-  real Tau[3], T1s[3];
-  if (change) {
-    const real q = fabs(Ts0) < RL(1e-1) ? 0.f : Tau_s / Ts0;
-#pragma unroll
-    for (int c = 0; c < 3; c++) { Tau[c] = Tau_n * vn[c] + q * Ts[c]; T1s[c] = (Tau[c] - T0[c]) * jacvec; }
-  } else {
-#pragma unroll
-    for (int c = 0; c < 3; c++) { Tau[c] = Tl[c]; T1s[c] = Tr[c]; }
-  }
-#pragma unroll
-  for (int c = 0; c < 3; c++) { F.scal[(FS_T1X + c) * ns + nd] = T1s[c]; X1[3][c] = T1s[c]; }
-  // the stage input level sees the new split-node traction before the volume
-  // kernel reads it (drv_rk_curv_col.cu:285, fault2wave on w_cur); no fault
-  // kernel reads the volume at i0
-  split_to_volume(g, cf, sc, ns, nd, i0, J, K, a.fc, T1s, const_cast<real *>(a.wcur));
-  {
-    const real s1[3] = { F.scal[FS_S1X * ns + nd], F.scal[FS_S1Y * ns + nd], F.scal[FS_S1Z * ns + nd] };
-    const real s2[3] = { F.scal[FS_S2X * ns + nd], F.scal[FS_S2Y * ns + nd], F.scal[FS_S2Z * ns + nd] };
-    const real tTs1 = Tau[0] * s1[0] + Tau[1] * s1[1] + Tau[2] * s1[2];
-    const real tTs2 = Tau[0] * s2[0] + Tau[1] * s2[1] + Tau[2] * s2[2];
-    real *Tn = F.out + CGFD_FAULT_TN * ns + nd, *T1o = F.out + CGFD_FAULT_TS1 * ns + nd, *T2o = F.out + CGFD_FAULT_TS2 * ns + nd;
-    if (a.mode == RK_FIRST) { *Tn = a.rkb * Tau_n; *T1o = a.rkb * tTs1; *T2o = a.rkb * tTs2; }
-    else { *Tn += a.rkb * Tau_n; *T1o += a.rkb * tTs1; *T2o += a.rkb * tTs2; }
-  }
-
-  // split-node velocity RHS and RK update (the output levels only; the
-  // stress kernel of this stage reads the fault velocity of the input level)
-  long o[6];
-  real hv[6];
-#pragma unroll
-  for (int m = 0; m < 2; m++) {
-    const real rr = 1.0f / ((m ? rho1 : rho0) * jac0);
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const real dx = m == 0 ? (kA0 * X1[3][c] - kA1 * X1[2][c] - kA2 * X1[1][c] - kA3 * X1[0][c])
-                              : (-kA0 * X1[3][c] + kA1 * X1[4][c] + kA2 * X1[5][c] + kA3 * X1[6][c]);
-      hv[3 * m + c] = (dx + DyT2[m][c] + DzT3[m][c]) * rr;
-      o[3 * m + c] = fidx(FVX + c, m, ns, nd);
-    }
-  }
-  rk_put_n<6>(a.mode, a.ca, a.cb, a.fc, a.fp, a.fo, a.fe, o, hv);
 }
 
 // x offset from the fault of slab slot y = 0..5: -3, -2, -1, 1, 2, 3
@@ -545,234 +403,334 @@ __device__ __forceinline__ void slab_stress(const FaultArgs &a, int j, int k, in
 }
 
 // ---------------------------------------------------------------------------
-// split nodes, one thread per node: velocity gradients of both sides
-// (continuity matrices or traction rate, free-surface rows), fault traction
-// rates and their RK update, the split-node volume point of the output
-// level, and after the last stage slip / slip rate / rupture time
+// row c of a 3x3 matrix times a vector held in shared memory, entries `st`
+// apart
+__device__ __forceinline__ real row3(const real *__restrict__ m, int c, const real *v, int st) {
+  return __ldg(m + 3 * c) * v[0] + __ldg(m + 3 * c + 1) * v[st] + __ldg(m + 3 * c + 2) * v[2 * st];
+}
+
+// split nodes: trial traction and linear slip-weakening friction
+// (trial_slipweakening_gpu), the stage traction output, the refresh of the
+// stage input's split-node volume point, the split-node velocity RHS with
+// its RK update; velocity gradients of both sides (continuity matrices or
+// traction rate, free-surface rows), fault traction rates and their RK
+// update, the split-node volume point of the output level, and after the
+// last stage slip / slip rate / rupture time
 // (sv_curv_col_el_iso_rhs_fault_stress_F_gpu :432-1159 / _B_gpu :1162-1879,
-// split nodes; fault2wave_gpu; fault_var_update_gpu)
-__device__ __forceinline__ void split_node(const FaultArgs &a, int j, int k, uint8_t fl) {
+// split nodes; fault2wave_gpu; fault_var_update_gpu).
+//
+// A block is 32 nodes of one row by six warps, one per side and component:
+// a lane holds one of the node's six velocities, T2 and T3, and the warps
+// meet through shared memory where a component needs the others (the
+// friction law, which every warp evaluates for itself, and the 3x3
+// matrices, of which each warp reads its row).  The kernel is bound by the
+// latency of its dependent loads: with one thread per node, 154 registers and
+// a chain of a hundred loads, a launch of 3200 nodes took 26.9 us on 25 of
+// the 148 SMs.
+__global__ void __launch_bounds__(192) k_fault_split(const FaultArgs a) {
+  enum { S_R = 0, S_VP, S_V, S_T2, S_T3, S_SY, S_SZ, S_SX, S_NV, S_N2, S_N3, S_N };
+  __shared__ real sh[S_N][6][32];
   const Grid &g = a.g;
-  const int J = j + NG, K = k + NG;
-  const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny, sc = g.scmp;
   const FaultDev &F = a.F;
-  const int i0 = F.i0;
-  const real *w = a.wcur;
-  const long ny = g.ny;
+  const int tx = threadIdx.x, q = threadIdx.y, m = q / 3, c = q - 3 * m;
+  const int j = a.j0 + blockIdx.x * 32 + tx, k = a.k0 + blockIdx.y;
+  const int J = j + NG, K = k + NG;
+  const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny, ny = g.ny, sc = g.scmp;
+  const uint8_t fl = j < a.j0 + a.nj ? F.flag[nd] : 0;
+  const bool act = fl & FL_SPLIT;
+  const int i0 = F.i0, mode = a.mode;
   const int km = g.nk - (k + 1);
-  const bool fwd = a.idir == 1;
-  const bool top = a.isfree && km == 0;
-  // fault velocity of each side, input level: fV[m][c]
-  real fV[2][3];
+  const bool fwd = a.idir == 1, top = a.isfree && km == 0;
+  const long p0 = g.at(i0, J, K);
+  const real *cf = a.coef;
+  // entries of this node: side and component e / of side s, component 0 (the
+  // components follow 32 apart)
+  auto S = [&](int n, int e) -> real & { return sh[n][e][tx]; };
+  const int sg = 2 * m - 1;
+  real x1 = 0.f, x2 = 0.f, x3 = 0.f, dy2 = 0.f, dz3 = 0.f;
+  real jac0 = 0.f, rho0 = 0.f, rho1 = 0.f, slip = 0.f, mus = 0.f, mud = 0.f, Dc = 1.f, C0 = 0.f;
+  real T0[3] = { 0.f, 0.f, 0.f }, dt1[3] = { 0.f, 0.f, 0.f };
+  real4 exi = make_real4(1.f, 0.f, 0.f, 0.f);
+  const long oV = fidx(FVX + c, m, ns, nd), o2 = fidx(FT2X + c, m, ns, nd), o3 = fidx(FT3X + c, m, ns, nd);
+  real uV = 0.f, u2 = 0.f, u3 = 0.f;       // what the RK updates start from
+  real cV = 0.f, c2 = 0.f, c3 = 0.f;       // stage input
+  if (act) {
+    // T1 = J e_xi . sigma at this side's i0+-1..3
+    const long pl = (long)a.tnj * a.tnk * 12;
+    const real *tr = a.trac + ((long)(K - a.tk0) * a.tnj + (J - a.tj0)) * 12 + c * pl;
+    x1 = tr[trac_slot(sg)]; x2 = tr[trac_slot(2 * sg)]; x3 = tr[trac_slot(3 * sg)];
+    // along-fault derivatives of the fault tractions and velocity
+    const real *t2 = a.fc + o2, *t3 = a.fc + o3, *v = a.fc + oV;
+    dy2 = (fl & FL_RUPY) ? mac22(t2, 1, a.jdir) : drp_rt(t2, 1, a.jdir);
+    if (a.isfree && km <= 3) {
+      // traction image of T3 about the free surface
+      real l[7];
 #pragma unroll
-  for (int c = 0; c < 3; c++) { fV[0][c] = a.fc[fidx(FVX + c, 0, ns, nd)]; fV[1][c] = a.fc[fidx(FVX + c, 1, ns, nd)]; }
-
-  // along-fault velocity derivatives of each side
-  real Sx[2][3], Sy[2][3], Sz[2][3];
-#pragma unroll
-  for (int m = 0; m < 2; m++) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const real *v = a.fc + fidx(FVX + c, m, ns, nd);
-      Sy[m][c] = (fl & FL_RUPY) ? mac22(v, 1, a.jdir) : drp_rt(v, 1, a.jdir);
-      if (a.isfree && km == 1) Sz[m][c] = mac22(v, ny, a.kdir);
-      else if (a.isfree && km == 2) Sz[m][c] = mac24(v, ny, a.kdir);
-      else Sz[m][c] = (fl & FL_RUPZ) ? mac22(v, ny, a.kdir) : drp_rt(v, ny, a.kdir);
-    }
-  }
-  const real *mat = F.mat;
-  auto M = [&](int id) { return mat + ((long)id * ns + nd) * 9; };
-  if (!top) {
-    if (a.imethod == 1) {
-      // one side from its one-sided difference, the other from continuity
-      // of traction rate across the fault
-      real o1[3], o2[3], o3[3], o4[3], o5[3];
-      if (fwd) {
-        const long q = g.at(i0 + 1, J, K);
-#pragma unroll
-        for (int c = 0; c < 3; c++) Sx[1][c] = w[g.w(VX + c, q)] - fV[1][c];
-        mv3(M(FM_P2M1), Sx[1], o1); mv3(M(FM_P2M2), Sy[1], o2); mv3(M(FM_P2M3), Sz[1], o3);
-        mv3(M(FM_P2M4), Sy[0], o4); mv3(M(FM_P2M5), Sz[0], o5);
-#pragma unroll
-        for (int c = 0; c < 3; c++) Sx[0][c] = o1[c] + o2[c] + o3[c] - o4[c] - o5[c];
-      } else {
-        const long q = g.at(i0 - 1, J, K);
-#pragma unroll
-        for (int c = 0; c < 3; c++) Sx[0][c] = fV[0][c] - w[g.w(VX + c, q)];
-        mv3(M(FM_M2P1), Sx[0], o1); mv3(M(FM_M2P2), Sy[0], o2); mv3(M(FM_M2P3), Sz[0], o3);
-        mv3(M(FM_M2P4), Sy[1], o4); mv3(M(FM_M2P5), Sz[1], o5);
-#pragma unroll
-        for (int c = 0; c < 3; c++) Sx[1][c] = o1[c] + o2[c] + o3[c] - o4[c] - o5[c];
-      }
+      for (int n = 0; n < 7; n++) l[n] = __ldg(t3 + (long)(n - 3) * ny);
+      odd_image(l, km + 3);
+      dz3 = drp_v(l + 3, a.kdir);
     } else {
-      // normal derivative of each side from the traction rate
-      real dt1[3] = { 0.f, 0.f, 0.f };
-      if (fl & FL_GRID) { dt1[0] = F.scal[FS_HT1X * ns + nd]; dt1[1] = F.scal[FS_HT1Y * ns + nd]; dt1[2] = F.scal[FS_HT1Z * ns + nd]; }
-      real o1[3], o2[3], o3[3];
-      mv3(M(FM_T1VXPLUS), dt1, o1); mv3(M(FM_VYVXPLUS), Sy[1], o2); mv3(M(FM_VZVXPLUS), Sz[1], o3);
-#pragma unroll
-      for (int c = 0; c < 3; c++) Sx[1][c] = o1[c] - o2[c] - o3[c];
-      mv3(M(FM_T1VXMIN), dt1, o1); mv3(M(FM_VYVXMIN), Sy[0], o2); mv3(M(FM_VZVXMIN), Sz[0], o3);
-#pragma unroll
-      for (int c = 0; c < 3; c++) Sx[0][c] = o1[c] - o2[c] - o3[c];
+      dz3 = (fl & FL_RUPZ) ? mac22(t3, ny, a.kdir) : drp_rt(t3, ny, a.kdir);
     }
-  } else {
-    // split nodes on the free surface: traction-free top as well
-    auto FM = [&](int id) { return F.fmat + ((long)id * ny + J) * 9; };
-    real o1[3], o2[3], o3[3];
-    if (a.imethod == 1) {
-      if (fwd) {
-        const long q = g.at(i0 + 1, J, K);
+    S(S_SY, q) = (fl & FL_RUPY) ? mac22(v, 1, a.jdir) : drp_rt(v, 1, a.jdir);
+    real dz;
+    if (a.isfree && km == 1) dz = mac22(v, ny, a.kdir);
+    else if (a.isfree && km == 2) dz = mac24(v, ny, a.kdir);
+    else dz = (fl & FL_RUPZ) ? mac22(v, ny, a.kdir) : drp_rt(v, ny, a.kdir);
+    S(S_SZ, q) = dz;
+    cV = __ldg(v); c2 = __ldg(t2); c3 = __ldg(t3);
+    if (mode != RK_FIRST) {
+      const real *l = mode == RK_LAST ? a.fe : a.fp;
+      uV = l[oV]; u2 = l[o2]; u3 = l[o3];
+    }
+    S(S_VP, q) = mode == RK_FIRST ? cV : (mode == RK_LAST ? a.fp[oV] : uV);
+    S(S_V, q) = cV; S(S_T2, q) = c2; S(S_T3, q) = c3;
+    const real img = kA1 * x1 + kA2 * x2 + kA3 * x3;
+    S(S_R, q) = 0.5f * ((real)sg * img + (dy2 + dz3));
+    // what the friction law reads of this node
+    jac0 = coef_jac(cf, p0);
+    exi = coef_row(cf, sc, 0, p0);
+    rho0 = F.scal[FS_RHO0 * ns + nd]; rho1 = F.scal[FS_RHO1 * ns + nd];
+    slip = F.out[CGFD_FAULT_SLIP * ns + nd];
+    mus = F.scal[FS_MUS * ns + nd]; mud = F.scal[FS_MUD * ns + nd];
+    Dc = F.scal[FS_DC * ns + nd]; C0 = F.scal[FS_C0 * ns + nd];
 #pragma unroll
-        for (int c = 0; c < 3; c++) Sx[1][c] = w[g.w(VX + c, q)] - fV[1][c];
-        mv3(FM(FF_P2M1), Sx[1], o1); mv3(FM(FF_P2M2), Sy[1], o2); mv3(FM(FF_P2M3), Sy[0], o3);
+    for (int n = 0; n < 3; n++) T0[n] = F.scal[(FS_T0X + n) * ns + nd];
+    if (a.imethod == 2 && (fl & FL_GRID)) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) Sx[0][c] = o1[c] + o2[c] - o3[c];
-      } else {
-        const long q = g.at(i0 - 1, J, K);
+      for (int n = 0; n < 3; n++) dt1[n] = F.scal[(FS_HT1X + n) * ns + nd];
+    }
+  }
+  __syncthreads();
+
+  real T1s[3] = { 0.f, 0.f, 0.f };
+  if (act) {
+    // trial traction from the velocity jump of time level n and friction
+    const real M0 = 0.5f * jac0 * rho0, M1 = 0.5f * jac0 * rho1;
+    real Tr[3];
 #pragma unroll
-        for (int c = 0; c < 3; c++) Sx[0][c] = fV[0][c] - w[g.w(VX + c, q)];
-        mv3(FM(FF_M2P1), Sx[0], o1); mv3(FM(FF_M2P2), Sy[0], o2); mv3(FM(FF_M2P3), Sy[1], o3);
+    for (int n = 0; n < 3; n++) {
+      const real dV = S(S_VP, 3 + n) - S(S_VP, n);
+      Tr[n] = 2.0f * (M0 * M1 * dV / a.dt + M0 * S(S_R, 3 + n) - M1 * S(S_R, n)) / (kA0 * (M0 + M1));
+    }
+    real vn[3] = { exi.x, exi.y, exi.z };
+    const real vn0 = sqrt(vn[0] * vn[0] + vn[1] * vn[1] + vn[2] * vn[2]);
+    const real jacvec = jac0 * vn0;
+    vn[0] /= vn0; vn[1] /= vn0; vn[2] /= vn0;
+    real Tl[3];
 #pragma unroll
-        for (int c = 0; c < 3; c++) Sx[1][c] = o1[c] + o2[c] - o3[c];
-      }
+    for (int n = 0; n < 3; n++) Tl[n] = Tr[n] / jacvec + T0[n];
+    const real Tn0 = Tl[0] * vn[0] + Tl[1] * vn[1] + Tl[2] * vn[2];
+    const real Ts[3] = { Tl[0] - vn[0] * Tn0, Tl[1] - vn[1] * Tn0, Tl[2] - vn[2] * Tn0 };
+    const real Ts0 = sqrt(Ts[0] * Ts[0] + Ts[1] * Ts[1] + Ts[2] * Ts[2]);
+    bool change = false;
+    real Tau_n = Tn0;
+    if (Tn0 >= 0.f) { Tau_n = 0.f; change = true; }     // the fault cannot open
+    const real fr = slip <= Dc ? mus - (mus - mud) * slip / Dc : mud;
+    const real Tau_c = -fr * Tau_n + C0;
+    real Tau_s = Ts0;
+    if (Ts0 >= Tau_c) { Tau_s = Tau_c; change = true; }
+    real Tau[3];
+    if (change) {
+      const real r = fabs(Ts0) < RL(1e-1) ? 0.f : Tau_s / Ts0;
+#pragma unroll
+      for (int n = 0; n < 3; n++) { Tau[n] = Tau_n * vn[n] + r * Ts[n]; T1s[n] = (Tau[n] - T0[n]) * jacvec; }
     } else {
-      real dt1[3] = { 0.f, 0.f, 0.f };
-      if (fl & FL_GRID) { dt1[0] = F.scal[FS_HT1X * ns + nd]; dt1[1] = F.scal[FS_HT1Y * ns + nd]; dt1[2] = F.scal[FS_HT1Z * ns + nd]; }
-      mv3(FM(FF_T1VXPLUS), dt1, o1); mv3(FM(FF_VYVXPLUS), Sy[1], o2);
 #pragma unroll
-      for (int c = 0; c < 3; c++) Sx[1][c] = o1[c] - o2[c];
-      mv3(FM(FF_T1VXMIN), dt1, o1); mv3(FM(FF_VYVXMIN), Sy[0], o2);
-#pragma unroll
-      for (int c = 0; c < 3; c++) Sx[0][c] = o1[c] - o2[c];
+      for (int n = 0; n < 3; n++) { Tau[n] = Tl[n]; T1s[n] = Tr[n]; }
     }
-    mv3(FM(FF_VX2VZ2), Sx[1], o1); mv3(FM(FF_VY2VZ2), Sy[1], o2);
+    if (q == 0) {
 #pragma unroll
-    for (int c = 0; c < 3; c++) Sz[1][c] = o1[c] + o2[c];
-    mv3(FM(FF_VX2VZ1), Sx[0], o1); mv3(FM(FF_VY2VZ1), Sy[0], o2);
+      for (int n = 0; n < 3; n++) F.scal[(FS_T1X + n) * ns + nd] = T1s[n];
+    } else if (q == 1) {
+      // the stage input level sees the new split-node traction before the
+      // volume kernel reads it (drv_rk_curv_col.cu:285, fault2wave on
+      // w_cur); no fault kernel reads the volume at i0
+      split_to_volume(g, cf, i0, J, K, &S(S_V, 0), &S(S_T2, 0), &S(S_T3, 0), 32, T1s, const_cast<real *>(a.wcur));
+    } else if (q == 2) {
+      const real s1[3] = { F.scal[FS_S1X * ns + nd], F.scal[FS_S1Y * ns + nd], F.scal[FS_S1Z * ns + nd] };
+      const real s2[3] = { F.scal[FS_S2X * ns + nd], F.scal[FS_S2Y * ns + nd], F.scal[FS_S2Z * ns + nd] };
+      const real t[3] = { Tau_n, Tau[0] * s1[0] + Tau[1] * s1[1] + Tau[2] * s1[2],
+                          Tau[0] * s2[0] + Tau[1] * s2[1] + Tau[2] * s2[2] };
+      // Tn, Ts1, Ts2 follow one another
+      real o[3] = { 0.f, 0.f, 0.f };
+      if (mode != RK_FIRST) {
 #pragma unroll
-    for (int c = 0; c < 3; c++) Sz[0][c] = o1[c] + o2[c];
-  }
-
-  // fault traction rates and RK update of T2, T3 on both sides
-  {
-    long o[12];
-    real h[12];
+        for (int n = 0; n < 3; n++) o[n] = F.out[(CGFD_FAULT_TN + n) * ns + nd];
+      }
 #pragma unroll
-    for (int m = 0; m < 2; m++) {
-      const int b2 = m ? FM_D21_2 : FM_D21_1, b3 = m ? FM_D31_2 : FM_D31_1;
-      real g1[3], g2[3], g3[3];
-      mv3(M(b2), Sx[m], g1); mv3(M(b2 + 1), Sy[m], g2); mv3(M(b2 + 2), Sz[m], g3);
-#pragma unroll
-      for (int c = 0; c < 3; c++) { h[6 * m + c] = g1[c] + g2[c] + g3[c]; o[6 * m + c] = fidx(FT2X + c, m, ns, nd); }
-      mv3(M(b3), Sx[m], g1); mv3(M(b3 + 1), Sy[m], g2); mv3(M(b3 + 2), Sz[m], g3);
-#pragma unroll
-      for (int c = 0; c < 3; c++) { h[6 * m + 3 + c] = g1[c] + g2[c] + g3[c]; o[6 * m + 3 + c] = fidx(FT3X + c, m, ns, nd); }
+      for (int n = 0; n < 3; n++) F.out[(CGFD_FAULT_TN + n) * ns + nd] = mode == RK_FIRST ? a.rkb * t[n] : o[n] + a.rkb * t[n];
     }
-    rk_put_n<12>(a.mode, a.ca, a.cb, a.fc, a.fp, a.fo, a.fe, o, h);
-  }
+    // split-node velocity RHS and RK update (the output levels only: the
+    // velocity taps of this stage read the input level)
+    const real rr = 1.0f / ((m ? rho1 : rho0) * jac0);
+    const real T1c = c == 0 ? T1s[0] : (c == 1 ? T1s[1] : T1s[2]);
+    const real dx = m == 0 ? (kA0 * T1c - kA1 * x1 - kA2 * x2 - kA3 * x3) : (-kA0 * T1c + kA1 * x1 + kA2 * x2 + kA3 * x3);
+    S(S_NV, q) = rk_put(mode, a.ca, a.cb, uV, cV, (dx + dy2 + dz3) * rr, a.fo + oV, a.fe + oV);
 
-  // the split-node volume point of the output level from the fault fields
-  {
-    const bool last = a.mode == RK_LAST;
-    const real T1s[3] = { F.scal[FS_T1X * ns + nd], F.scal[FS_T1Y * ns + nd], F.scal[FS_T1Z * ns + nd] };
-    split_to_volume(g, a.coef, sc, ns, nd, i0, J, K, last ? a.fe : a.fo, T1s, last ? a.wend : a.wout);
-  }
-
-  // end of step: slip rate, slip, traction rate, peak slip rate, rupture time
-  if (a.mode == RK_LAST) {
-    const real *f = a.fe;
-    const real s1[3] = { F.scal[FS_S1X * ns + nd], F.scal[FS_S1Y * ns + nd], F.scal[FS_S1Z * ns + nd] };
-    const real s2[3] = { F.scal[FS_S2X * ns + nd], F.scal[FS_S2Y * ns + nd], F.scal[FS_S2Z * ns + nd] };
-    real dV[3];
+    // normal velocity derivative of this side
+    const int me = 3 * m, ot = 3 - me;
+    real sx;
+    if (a.imethod == 1 && m == (fwd ? 1 : 0)) {
+      // its one-sided difference
+      const real *w = a.wcur;
+      sx = fwd ? w[g.w(VX + c, g.at(i0 + 1, J, K))] - cV : cV - w[g.w(VX + c, g.at(i0 - 1, J, K))];
+    } else if (a.imethod == 1) {
+      // continuity of the traction rate across the fault, from the other
+      // side's one-sided difference
+      const real4 w1 = __ldg(reinterpret_cast<const real4 *>(a.wcur) + g.at(fwd ? i0 + 1 : i0 - 1, J, K));
+      const real wv[3] = { w1.x, w1.y, w1.z };
+      real d[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) dV[c] = f[fidx(FVX + c, 1, ns, nd)] - f[fidx(FVX + c, 0, ns, nd)];
+      for (int n = 0; n < 3; n++) d[n] = fwd ? wv[n] - S(S_V, ot + n) : S(S_V, ot + n) - wv[n];
+      if (!top) {
+        auto M = [&](int id) { return F.mat + ((long)id * ns + nd) * 9; };
+        const int b = fwd ? FM_P2M1 : FM_M2P1;
+        sx = row3(M(b), c, d, 1) + row3(M(b + 1), c, &S(S_SY, ot), 32) + row3(M(b + 2), c, &S(S_SZ, ot), 32) -
+             row3(M(b + 3), c, &S(S_SY, me), 32) - row3(M(b + 4), c, &S(S_SZ, me), 32);
+      } else {
+        auto FM = [&](int id) { return F.fmat + ((long)id * ny + J) * 9; };
+        const int b = fwd ? FF_P2M1 : FF_M2P1;
+        sx = row3(FM(b), c, d, 1) + row3(FM(b + 1), c, &S(S_SY, ot), 32) - row3(FM(b + 2), c, &S(S_SY, me), 32);
+      }
+    } else if (!top) {
+      // from the traction rate
+      auto M = [&](int id) { return F.mat + ((long)id * ns + nd) * 9; };
+      const int b = m ? FM_T1VXPLUS : FM_T1VXMIN;
+      sx = row3(M(b), c, dt1, 1) - row3(M(b + 1), c, &S(S_SY, me), 32) - row3(M(b + 2), c, &S(S_SZ, me), 32);
+    } else {
+      auto FM = [&](int id) { return F.fmat + ((long)id * ny + J) * 9; };
+      const int b = m ? FF_T1VXPLUS : FF_T1VXMIN;
+      sx = row3(FM(b), c, dt1, 1) - row3(FM(b + 1), c, &S(S_SY, me), 32);
+    }
+    S(S_SX, q) = sx;
+  }
+  __syncthreads();
+
+  // fault traction rates and RK update of T2, T3
+  if (act) {
+    const int me = 3 * m;
+    real z[3];
+    if (top) {
+      // split nodes on the free surface: traction-free top as well
+      const real *A = F.fmat + ((long)(m ? FF_VX2VZ2 : FF_VX2VZ1) * ny + J) * 9, *B = A + ny * 9;
+#pragma unroll
+      for (int n = 0; n < 3; n++) z[n] = row3(A, n, &S(S_SX, me), 32) + row3(B, n, &S(S_SY, me), 32);
+    } else {
+#pragma unroll
+      for (int n = 0; n < 3; n++) z[n] = S(S_SZ, me + n);
+    }
+    const real *D2 = F.mat + ((long)(m ? FM_D21_2 : FM_D21_1) * ns + nd) * 9, *D3 = D2 + 27 * ns;
+    const real h2 = row3(D2, c, &S(S_SX, me), 32) + row3(D2 + 9 * ns, c, &S(S_SY, me), 32) + row3(D2 + 18 * ns, c, z, 1);
+    const real h3 = row3(D3, c, &S(S_SX, me), 32) + row3(D3 + 9 * ns, c, &S(S_SY, me), 32) + row3(D3 + 18 * ns, c, z, 1);
+    S(S_N2, q) = rk_put(mode, a.ca, a.cb, u2, c2, h2, a.fo + o2, a.fe + o2);
+    S(S_N3, q) = rk_put(mode, a.ca, a.cb, u3, c3, h3, a.fo + o3, a.fe + o3);
+  }
+  __syncthreads();
+  if (!act) return;
+
+  if (q == 0) {
+    // the split-node volume point of the output level
+    split_to_volume(g, cf, i0, J, K, &S(S_NV, 0), &S(S_N2, 0), &S(S_N3, 0), 32, T1s, mode == RK_LAST ? a.wend : a.wout);
+  } else if (mode == RK_LAST && q == 1) {
+    // end of step: slip rate, slip, peak slip rate, rupture time
+    real s1[3], s2[3], dV[3];
+#pragma unroll
+    for (int n = 0; n < 3; n++) {
+      s1[n] = F.scal[(FS_S1X + n) * ns + nd];
+      s2[n] = F.scal[(FS_S2X + n) * ns + nd];
+      dV[n] = S(S_NV, 3 + n) - S(S_NV, n);
+    }
     const real Vs1 = dV[0] * s1[0] + dV[1] * s1[1] + dV[2] * s1[2];
     const real Vs2 = dV[0] * s2[0] + dV[1] * s2[1] + dV[2] * s2[2];
     const real Vs = sqrt(Vs2 * Vs2 + Vs1 * Vs1);
     real *o = F.out;
+    const real l0 = slip, l1 = o[CGFD_FAULT_SLIP1 * ns + nd], l2 = o[CGFD_FAULT_SLIP2 * ns + nd];
+    const real pk = o[CGFD_FAULT_PEAK_VS * ns + nd];
     o[CGFD_FAULT_VS * ns + nd] = Vs;
     o[CGFD_FAULT_VS1 * ns + nd] = Vs1;
     o[CGFD_FAULT_VS2 * ns + nd] = Vs2;
-    o[CGFD_FAULT_SLIP * ns + nd] += Vs * a.dt;
-    o[CGFD_FAULT_SLIP1 * ns + nd] += Vs1 * a.dt;
-    o[CGFD_FAULT_SLIP2 * ns + nd] += Vs2 * a.dt;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const real t1 = F.scal[(FS_T1X + c) * ns + nd];
-      F.scal[(FS_HT1X + c) * ns + nd] = (t1 - F.scal[(FS_MT1X + c) * ns + nd]) / a.dt;
-      F.scal[(FS_MT1X + c) * ns + nd] = t1;
-    }
-    if (Vs > o[CGFD_FAULT_PEAK_VS * ns + nd]) o[CGFD_FAULT_PEAK_VS * ns + nd] = Vs;
-    uint8_t fl2 = F.flag[nd];
-    if (!(fl2 & FL_T0SET) && Vs > RL(1e-3)) {
+    o[CGFD_FAULT_SLIP * ns + nd] = l0 + Vs * a.dt;
+    o[CGFD_FAULT_SLIP1 * ns + nd] = l1 + Vs1 * a.dt;
+    o[CGFD_FAULT_SLIP2 * ns + nd] = l2 + Vs2 * a.dt;
+    if (Vs > pk) o[CGFD_FAULT_PEAK_VS * ns + nd] = Vs;
+    if (!(fl & FL_T0SET) && Vs > RL(1e-3)) {
       o[CGFD_FAULT_INIT_T0 * ns + nd] = (a.ctl->it + 1) * a.dt;
-      F.flag[nd] = fl2 | FL_T0SET;
+      F.flag[nd] = fl | FL_T0SET;
     }
     if (!isfinite(Vs)) atomicOr(&a.ctl->err, 1);
+  } else if (mode == RK_LAST && q == 2) {
+    // traction rate of the step
+    real mt[3];
+#pragma unroll
+    for (int n = 0; n < 3; n++) mt[n] = F.scal[(FS_MT1X + n) * ns + nd];
+#pragma unroll
+    for (int n = 0; n < 3; n++) {
+      F.scal[(FS_HT1X + n) * ns + nd] = (T1s[n] - mt[n]) / a.dt;
+      F.scal[(FS_MT1X + n) * ns + nd] = T1s[n];
+    }
   }
 }
 
-// ---------------------------------------------------------------------------
-// split nodes, one thread per node: the trial traction and friction, then
-// the traction rates, the split-node volume point of the output level and
-// (after the last stage) slip and slip rate, in one pass.  The second part
-// reads the traction this thread's first part wrote, the stage input at
-// i0 +- 1 and the fault fields of the input level, none of which a split
-// node's first part changes for another node, so one thread can do both.
-__global__ void __launch_bounds__(128) k_fault_split(const FaultArgs a) {
-  const int j = a.j0 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = a.k0 + blockIdx.y * blockDim.y + threadIdx.y;
-  if (j >= a.j0 + a.nj || k >= a.k0 + a.nk) return;
-  const uint8_t fl = a.F.flag[(j + NG) + (long)(k + NG) * a.g.ny];
-  if (!(fl & FL_SPLIT)) return;
-  split_trial(a, j, k, fl);
-  split_node(a, j, k, fl);
-}
-
-// the nine components of point p of a level (grouped layout)
-__device__ __forceinline__ void lev9(const real *w, long sc, long p, real v[9]) {
-  const real4 x = reinterpret_cast<const real4 *>(w)[p], y = reinterpret_cast<const real4 *>(w + 4 * sc)[p];
-  v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-  v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
-  v[8] = w[8 * sc + p];
-}
-// nine components to point p of a level, whole 16-byte groups
-__device__ __forceinline__ void put9(real *w, long sc, long p, const real v[9]) {
-  reinterpret_cast<real4 *>(w)[p] = make_real4(v[0], v[1], v[2], v[3]);
-  reinterpret_cast<real4 *>(w + 4 * sc)[p] = make_real4(v[4], v[5], v[6], v[7]);
-  w[8 * sc + p] = v[8];
-}
-
-// the six volume points i0-3..i0+3 (not i0) of split nodes, one thread per
-// point with the x offset fastest: velocity RHS (traction image through the
-// fault) and stress RHS (the fault's one-sided x operators), then the RK
-// update of all nine components with whole-group stores
-__global__ void __launch_bounds__(192) k_fault_slab(const FaultArgs a) {
+// the six volume points i0-3..i0+3 (not i0) of split nodes, x offset fastest:
+// velocity RHS (traction image through the fault) and stress RHS (the
+// fault's one-sided x operators), then the RK update with whole-group stores.
+// Two threads a point, one per RHS: the two read nothing of one another, and
+// the launch is as long as one thread's chain of loads where the fault does
+// not fill the GPU.  The halves meet in shared memory because the first
+// 16-byte group holds three velocities and Txx: the first half then updates
+// that group, the second (Tyy Tzz Tyz Txz) and Txy; each has asked for the
+// levels its update starts from before its RHS.
+constexpr int kSlabPoints = 96;
+__global__ void __launch_bounds__(2 * kSlabPoints) k_fault_slab(const FaultArgs a) {
+  __shared__ real sh[9][kSlabPoints];
   const Grid &g = a.g;
-  int j, k, s;
-  if (!slab_item(a, (long)blockIdx.x * blockDim.x + threadIdx.x, j, k, s)) return;
-  if (!(a.F.flag[(j + NG) + (long)(k + NG) * g.ny] & FL_SPLIT)) return;
-  real h[9];
-  slab_velocity(a, j, k, s, h);
-  slab_stress(a, j, k, s, h + 3);
-  const long q = g.at(a.F.i0 + s, j + NG, k + NG), sc = g.scmp;
-  real u[9], e[9], r[9];
-  if (a.mode != RK_THIRD) lev9(a.wcur, sc, q, u);
-  if (a.mode != RK_FIRST) lev9(a.mode == RK_LAST ? a.wend : a.wpre, sc, q, e);
-  if (a.mode == RK_LAST) {
+  const int tx = threadIdx.x, half = threadIdx.y, mode = a.mode;
+  int j = 0, k = 0, s = 1;
+  bool act = slab_item(a, (long)blockIdx.x * kSlabPoints + tx, j, k, s);
+  act = act && (a.F.flag[(j + NG) + (long)(k + NG) * g.ny] & FL_SPLIT);
+  const long sc = g.scmp, q = act ? g.at(a.F.i0 + s, j + NG, k + NG) : 0;
+  const long o4 = half ? 4 * sc + 4 * q : 4 * q, o1 = 8 * sc + q;
+  real4 cur = make_real4(0.f, 0.f, 0.f, 0.f), u0 = cur;
+  real cur1 = 0.f, u1 = 0.f;
+  if (act) {
+    const real *l = mode == RK_LAST ? a.wend : a.wpre;
+    if (mode != RK_THIRD) cur = *reinterpret_cast<const real4 *>(a.wcur + o4);
+    if (mode != RK_FIRST) u0 = *reinterpret_cast<const real4 *>(l + o4);
+    if (half) {
+      if (mode != RK_THIRD) cur1 = a.wcur[o1];
+      if (mode != RK_FIRST) u1 = l[o1];
+      real h[6];
+      slab_stress(a, j, k, s, h);
 #pragma unroll
-    for (int c = 0; c < 9; c++) r[c] = rk_end(e[c], u[c], a.cb * h[c]);
-    put9(a.wend, sc, q, r);
+      for (int n = 0; n < 6; n++) sh[3 + n][tx] = h[n];
+    } else {
+      real h[3];
+      slab_velocity(a, j, k, s, h);
+#pragma unroll
+      for (int n = 0; n < 3; n++) sh[n][tx] = h[n];
+    }
+  }
+  __syncthreads();
+  if (!act) return;
+  const int n0 = 4 * half;
+  const real h[4] = { sh[n0][tx], sh[n0 + 1][tx], sh[n0 + 2][tx], sh[n0 + 3][tx] };
+  if (mode == RK_LAST) {
+    *reinterpret_cast<real4 *>(a.wend + o4) =
+        make_real4(rk_end(u0.x, cur.x, a.cb * h[0]), rk_end(u0.y, cur.y, a.cb * h[1]),
+                   rk_end(u0.z, cur.z, a.cb * h[2]), rk_end(u0.w, cur.w, a.cb * h[3]));
+    if (half) a.wend[o1] = rk_end(u1, cur1, a.cb * sh[8][tx]);
     return;
   }
-#pragma unroll
-  for (int c = 0; c < 9; c++) r[c] = rk_out(a.mode == RK_FIRST ? u[c] : e[c], a.ca * h[c]);
-  put9(a.wout, sc, q, r);
-  if (a.mode == RK_SECOND) {
-#pragma unroll
-    for (int c = 0; c < 9; c++) r[c] = rk_v(e[c], u[c], a.ca * h[c]);
-    put9(a.wend, sc, q, r);
+  const real4 b = mode == RK_FIRST ? cur : u0;
+  *reinterpret_cast<real4 *>(a.wout + o4) = make_real4(rk_out(b.x, a.ca * h[0]), rk_out(b.y, a.ca * h[1]),
+                                                       rk_out(b.z, a.ca * h[2]), rk_out(b.w, a.ca * h[3]));
+  if (half) a.wout[o1] = rk_out(mode == RK_FIRST ? cur1 : u1, a.ca * sh[8][tx]);
+  if (mode == RK_SECOND) {
+    *reinterpret_cast<real4 *>(a.wend + o4) =
+        make_real4(rk_v(u0.x, cur.x, a.ca * h[0]), rk_v(u0.y, cur.y, a.ca * h[1]),
+                   rk_v(u0.z, cur.z, a.ca * h[2]), rk_v(u0.w, cur.w, a.ca * h[3]));
+    if (half) a.wend[o1] = rk_v(u1, cur1, a.ca * sh[8][tx]);
   }
 }
 
@@ -780,8 +738,7 @@ __global__ void __launch_bounds__(192) k_fault_slab(const FaultArgs a) {
 // stations and fault stations of the current level (io_recv_keep,
 // io_funcs.cu:428-469, including its use of corner 5 in place of corner 4;
 // io_fault_recv_keep, io_funcs.cu:2313-2351)
-__global__ void k_record(const StationArgs a) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void record_item(const StationArgs &a, int t) {
   const int rec = a.ctl->nrec;
   const StationDev &S = a.st;
   if (rec >= S.max_rec) return;
@@ -811,30 +768,46 @@ __global__ void k_record(const StationArgs a) {
   }
 }
 
+__global__ void __launch_bounds__(128) k_record(const __grid_constant__ StationArgs a) {
+  record_item(a, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// what a stage's split-node kernel needs first, in one launch (the three
+// parts read the stage input and write apart from one another): blocks of
+// welded nodes, of tractions, and in a step's first stage of station
+// samples, which precede everything that changes the sampled level and the
+// fault output.  Small grids are bound by the number of dependent launches:
+// a kernel of 4 us each for the two fault parts and 5 us for the stations
+// before, 5 us together.
+__global__ void __launch_bounds__(192) k_fault_pre(const __grid_constant__ FaultArgs a, const __grid_constant__ StationArgs st,
+                                                   int nweld, int ntrac) {
+  const int b = blockIdx.x;
+  if (b < nweld) weld_node(a, (long)b * 192 + threadIdx.x);
+  else if (b < nweld + ntrac) trac_item(a, (long)(b - nweld) * 192 + threadIdx.x);
+  else record_item(st, (b - nweld - ntrac) * 192 + threadIdx.x);
+}
+
 __global__ void k_advance(Ctl *c, int max_rec) {
   c->it += 1;
   if (c->nrec < max_rec) c->nrec += 1;
 }
 
 // ---------------------------------------------------------------------------
-// first part of a stage: welded nodes, tractions, trial traction and
-// friction (which also refreshes the stage input at i0, read by the volume
-// kernels); returns the number of launches
-int launch_fault_pre(const FaultArgs &a, cudaStream_t st) {
-  {
-    dim3 blk(32, 4), grd((a.wnj + 31) / 32, (a.wnk + 3) / 4);
-    k_fault_weld<<<grd, blk, 0, st>>>(a);
-  }
-  if (a.nj <= 0 || a.nk <= 0) return 1;
-  {
-    const long n = (long)a.tnj * a.tnk * 12;
-    k_fault_trac<<<(unsigned)((n + 191) / 192), 192, 0, st>>>(a);
-  }
-  {
-    dim3 blk(32, 4), grd((a.nj + 31) / 32, (a.nk + 3) / 4);
-    k_fault_split<<<grd, blk, 0, st>>>(a);
-  }
-  return 3;
+// first part of a stage: welded nodes, tractions (and, with st, the
+// stations), then trial traction and friction (which also refreshes the
+// stage input at i0, read by the volume kernels); returns the number of
+// launches
+int launch_fault_pre(const FaultArgs &a, const StationArgs *rec, cudaStream_t st) {
+  const bool split = a.nj > 0 && a.nk > 0;
+  const int nweld = (int)(((long)a.wnj * a.wnk + 191) / 192);
+  const int ntrac = split ? (int)(((long)a.tnj * a.tnk * 12 + 191) / 192) : 0;
+  const int nrec = rec ? ((rec->st.n + rec->st.nf) * 9 + 191) / 192 : 0;
+  const StationArgs none{};
+  k_fault_pre<<<nweld + ntrac + nrec, 192, 0, st>>>(a, rec ? *rec : none, nweld, ntrac);
+  if (!split) return 1;
+  const dim3 blk(32, 6), grd((a.nj + 31) / 32, a.nk);
+  k_fault_split<<<grd, blk, 0, st>>>(a);
+  return 2;
 }
 
 // second part: the slab points around the split nodes; independent of the
@@ -842,7 +815,7 @@ int launch_fault_pre(const FaultArgs &a, cudaStream_t st) {
 int launch_fault_post(const FaultArgs &a, cudaStream_t st) {
   if (a.nj <= 0 || a.nk <= 0) return 0;
   const long nslab = (long)a.nj * a.nk * 6;
-  k_fault_slab<<<(unsigned)((nslab + 191) / 192), 192, 0, st>>>(a);
+  k_fault_slab<<<(unsigned)((nslab + kSlabPoints - 1) / kSlabPoints), dim3(kSlabPoints, 2), 0, st>>>(a);
   return 1;
 }
 

@@ -98,30 +98,37 @@ constexpr int kTileX = 32, kTileY = 4;
 struct VolBox {
   int i0, i1, j0, j1, k0, k1;
   int nbx, nby, first;
+  int kind;
 };
+constexpr int kMaxBoxes = 48;
 
 struct VolArgs {
   Grid g;
   int nbox, nblocks;
   int ychunk;                  // interior kernel: y tiles per chunk (z marches within a chunk)
-  VolBox box[16];
+  VolBox box[kMaxBoxes];
   const real *cur, *pre;
   real *out, *end;            // next-stage level (null at the last stage), E
   const real *coef, *free_mat;   // packed metric and medium (coef_row / coef_jac)
   real ca, cb;
   int isfree;
   int nfault;
-  // 1: the interior kernel leaves the fault planes x = i0 within each
-  // fault's split box grown by 3 nodes (welded nodes too; ghost-inclusive
-  // J0, J1, K0, K1 in fdef) to a later launch, so that it reads nothing the
-  // stage's first fault kernels write and may run beside them; outside that
-  // box no tap of a plane point reaches a split node
+  // 1: the launch leaves the fault planes x = i0 within each fault's split
+  // box grown by 3 nodes (welded nodes too; ghost-inclusive J0, J1, K0, K1
+  // in fdef) to a later one, so that it reads nothing the stage's first
+  // fault kernels write and may run beside them; outside that box no tap of
+  // a plane point reaches a split node
   int defer_i0;
   int fi0[MAXF];
   int fdef[MAXF][4];
   const uint8_t *fflag[MAXF];
   PmlFaceDev pml[6];           // indexed 2*dim + side; `on` = 0 when absent
 };
+
+// operator triple N (4 x direction + 2 y + z) of the kernels that hold every
+// kind; each is defined in a unit of its own
+template <int N>
+void launch_volume_all_n(const VolArgs &a, int mode, cudaStream_t st);
 
 struct FaultArgs {
   Grid g;
@@ -178,6 +185,8 @@ struct PeakArgs {
   const real *wend, *wpre;
   real *pg, *dis;
   real dt;
+  Ctl *ctl;
+  int max_rec;
 };
 
 }  // namespace cgfd

@@ -344,12 +344,20 @@ enum { INTERIOR = 0, SHELL = 1, FACE_X = 2, FACE_Y = 3, FACE_Z = 4, EDGE = 5, PL
 // TOP: the shell's code without the PML faces, for the rows under the free
 // surface away from every PML face (fewer live values than the shell)
 
-// block -> point; boxes with a narrow x extent (PML x slabs) pack their
-// points densely instead of leaving most of a 32-wide row idle
-__device__ __forceinline__ bool locate(const VolArgs &a, int &i, int &j, int &k) {
-  int b = 0;
+// block -> box of a launch's list (sorted by first block)
+__device__ __forceinline__ int box_of_block(const VolArgs &a) {
+  int lo = 0, hi = a.nbox - 1;
 #pragma unroll 1
-  while (b + 1 < a.nbox && (int)blockIdx.x >= a.box[b + 1].first) b++;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if ((int)blockIdx.x >= a.box[mid].first) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+// block -> point of box b; boxes with a narrow x extent (PML x slabs) pack
+// their points densely instead of leaving most of a 32-wide row idle
+__device__ __forceinline__ bool locate(const VolArgs &a, int b, int &i, int &j, int &k) {
   const VolBox &B = a.box[b];
   const int bid = blockIdx.x - B.first;
   const int ni = B.i1 - B.i0 + 1, nj = B.j1 - B.j0 + 1;
@@ -373,7 +381,7 @@ __device__ __forceinline__ bool locate(const VolArgs &a, int &i, int &j, int &k)
 // chunks).  The blocks of one y chunk of a.ychunk tiles march up z before
 // the next chunk starts, so the planes a z window touches stay in L2 (a
 // whole xy plane per z row would need more than the 126 MB L2 holds).
-__device__ __forceinline__ bool locate_interior(const VolArgs &a, int &i, int &j, int &k) {
+[[maybe_unused]] __device__ __forceinline__ bool locate_interior(const VolArgs &a, int &i, int &j, int &k) {
   const VolBox &B = a.box[0];
   const int nkb = B.k1 - B.k0 + 1;
   const int chunk = blockIdx.z / nkb, bz = blockIdx.z - chunk * nkb;
@@ -386,13 +394,12 @@ __device__ __forceinline__ bool locate_interior(const VolArgs &a, int &i, int &j
 
 // points that another kernel updates: the split-node slabs (i0-3..i0+3 of
 // unwelded nodes) belong to the fault kernels; with defer_i0 the fault
-// planes go to the PLANE launch
-template <int KIND>
+// planes go to a later launch
 __device__ __forceinline__ bool other_kernels_point(const VolArgs &a, int I, int J, int K) {
   for (int f = 0; f < a.nfault; f++) {
     const int d = I - a.fi0[f];
     if (d < -3 || d > 3) continue;
-    if (KIND == INTERIOR && d == 0 && a.defer_i0 && J >= a.fdef[f][0] && J <= a.fdef[f][1] && K >= a.fdef[f][2] &&
+    if (d == 0 && a.defer_i0 && J >= a.fdef[f][0] && J <= a.fdef[f][1] && K >= a.fdef[f][2] &&
         K <= a.fdef[f][3])
       return true;
     if (__ldg(a.fflag[f] + J + (long)K * a.g.ny) & FL_SPLIT) return true;
@@ -424,19 +431,15 @@ __device__ __forceinline__ bool other_kernels_point(const VolArgs &a, int I, int
 #define CGFD_LB_FACE 6
 #endif
 
+// one RK stage of one point
 template <int ID, int JD, int KD, int MODE, int KIND>
-__global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? CGFD_LB_INTERIOR
-                                         : (KIND == SHELL || KIND == EDGE ? CGFD_LB_SHELL
-                                                                          : (KIND == TOP ? CGFD_LB_TOP : CGFD_LB_FACE)))
-    k_volume(const __grid_constant__ VolArgs a) {
+__device__ __forceinline__ void volume_point(const VolArgs &a, int i, int j, int k) {
   static_assert(KIND >= INTERIOR && KIND <= TOP, "kernel kind");
   const Grid &g = a.g;
   const long sc = g.scmp;
-  int i, j, k;
-  if (KIND == INTERIOR ? !locate_interior(a, i, j, k) : !locate(a, i, j, k)) return;
   const int I = i + NG, J = j + NG, K = k + NG;
   const long p = g.at(I, J, K);
-  if (other_kernels_point<KIND>(a, I, J, K)) return;
+  if (other_kernels_point(a, I, J, K)) return;
 #if CGFD_PREFETCH
   // the RK update reads the time-n level (in the last stage V) at its end:
   // ask L2 for its lines now, so that those reads wait on L2, not DRAM
@@ -620,6 +623,48 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
   rk_update<MODE>(a, p, v0, h);
 }
 
+template <int ID, int JD, int KD, int MODE, int KIND>
+__global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? CGFD_LB_INTERIOR
+                                         : (KIND == SHELL || KIND == EDGE ? CGFD_LB_SHELL
+                                                                          : (KIND == TOP ? CGFD_LB_TOP : CGFD_LB_FACE)))
+    k_volume(const __grid_constant__ VolArgs a) {
+  int i, j, k;
+  if (KIND == INTERIOR ? !locate_interior(a, i, j, k) : !locate(a, box_of_block(a), i, j, k)) return;
+  volume_point<ID, JD, KD, MODE, KIND>(a, i, j, k);
+}
+
+#ifndef CGFD_LB_ALL
+#define CGFD_LB_ALL 6
+#endif
+// every kind in one launch, each block the kind of its box (merge_points in
+// api.cu says when).  6 blocks per SM as the boundary kinds have them alone;
+// 5: 105 us per step of 36x56x32 and 419 of 101x163x77, 8: 116 and 433, 6: 107
+// and 420.
+template <int ID, int JD, int KD, int MODE>
+__global__ void __launch_bounds__(BX * BY, CGFD_LB_ALL) k_volume_all(const __grid_constant__ VolArgs a) {
+  const int b = box_of_block(a);
+  int i, j, k;
+  if (!locate(a, b, i, j, k)) return;
+  switch (a.box[b].kind) {
+    case INTERIOR: volume_point<ID, JD, KD, MODE, INTERIOR>(a, i, j, k); break;
+    case FACE_X: volume_point<ID, JD, KD, MODE, FACE_X>(a, i, j, k); break;
+    case FACE_Y: volume_point<ID, JD, KD, MODE, FACE_Y>(a, i, j, k); break;
+    case FACE_Z: volume_point<ID, JD, KD, MODE, FACE_Z>(a, i, j, k); break;
+    case EDGE: volume_point<ID, JD, KD, MODE, EDGE>(a, i, j, k); break;
+    case TOP: volume_point<ID, JD, KD, MODE, TOP>(a, i, j, k); break;
+    default: volume_point<ID, JD, KD, MODE, SHELL>(a, i, j, k); break;
+  }
+}
+
+template <int ID, int JD, int KD>
+void launch_all(const VolArgs &a, int mode, cudaStream_t st) {
+  const dim3 blk(BX, BY, 1);
+  if (mode == RK_FIRST) k_volume_all<ID, JD, KD, RK_FIRST><<<a.nblocks, blk, 0, st>>>(a);
+  else if (mode == RK_SECOND) k_volume_all<ID, JD, KD, RK_SECOND><<<a.nblocks, blk, 0, st>>>(a);
+  else if (mode == RK_THIRD) k_volume_all<ID, JD, KD, RK_THIRD><<<a.nblocks, blk, 0, st>>>(a);
+  else k_volume_all<ID, JD, KD, RK_LAST><<<a.nblocks, blk, 0, st>>>(a);
+}
+
 template <int ID, int JD, int KD, int KIND>
 void launch4(const VolArgs &a, int mode, cudaStream_t st) {
   if (a.nbox == 0) return;
@@ -654,37 +699,52 @@ void launch_kind(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaS
 
 // This file is compiled once per kernel kind (CGFD_VOLUME_KIND = 0..7, set
 // by the build) so that the 32 instantiations of each kind build in
-// parallel; unit 0 also holds the host helpers.
+// parallel, and once per operator triple for the kernels that hold every
+// kind (8..15); unit 0 also holds the host helpers.
 #ifndef CGFD_VOLUME_KIND
 #define CGFD_VOLUME_KIND 0
 #endif
 
 #if CGFD_VOLUME_KIND == 0
-// boxes (interior indices, inclusive) -> block layout of one launch; with
-// pack, boxes at most 24 points wide in x are packed (nbx = 0); the
-// interior kernel's 3-D grid needs the tiled layout (pack = false)
-void volume_boxes(VolArgs &a, const int (*boxes)[6], int n, bool pack) {
-  a.nbox = 0;
-  int first = 0;
+// append n boxes (interior indices, inclusive) of one kind to a launch's
+// list; with pack, boxes at most 24 points wide are packed (nbx = 0); the
+// interior kernel's 3-D grid needs the tiled layout (pack = false).  False
+// when the list is full.
+bool volume_boxes(VolArgs &a, int kind, const int (*boxes)[6], int n, bool pack) {
   for (int q = 0; q < n; q++) {
     const int *b = boxes[q];
     if (b[1] < b[0] || b[3] < b[2] || b[5] < b[4]) continue;
+    if (a.nbox >= kMaxBoxes) return false;
     VolBox &B = a.box[a.nbox++];
     B.i0 = b[0]; B.i1 = b[1]; B.j0 = b[2]; B.j1 = b[3]; B.k0 = b[4]; B.k1 = b[5];
+    B.kind = kind;
+    B.first = a.nblocks;
     const int ni = b[1] - b[0] + 1, nj = b[3] - b[2] + 1, nk = b[5] - b[4] + 1;
     if (pack && ni <= 24) {
       B.nbx = 0;
       B.nby = (ni * nj + BX * BY - 1) / (BX * BY);
-      B.first = first;
-      first += B.nby * nk;
+      a.nblocks += B.nby * nk;
     } else {
       B.nbx = (ni + BX - 1) / BX;
       B.nby = (nj + BY - 1) / BY;
-      B.first = first;
-      first += B.nbx * B.nby * nk;
+      a.nblocks += B.nbx * B.nby * nk;
     }
   }
-  a.nblocks = first;
+  return true;
+}
+
+void launch_volume_all(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st) {
+  if (a.nbox == 0) return;
+  switch (idir * 4 + jdir * 2 + kdir) {
+    case 0: launch_volume_all_n<0>(a, mode, st); break;
+    case 1: launch_volume_all_n<1>(a, mode, st); break;
+    case 2: launch_volume_all_n<2>(a, mode, st); break;
+    case 3: launch_volume_all_n<3>(a, mode, st); break;
+    case 4: launch_volume_all_n<4>(a, mode, st); break;
+    case 5: launch_volume_all_n<5>(a, mode, st); break;
+    case 6: launch_volume_all_n<6>(a, mode, st); break;
+    default: launch_volume_all_n<7>(a, mode, st); break;
+  }
 }
 
 void launch_volume_interior(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st) {
@@ -714,9 +774,15 @@ void launch_volume_edge(const VolArgs &a, int idir, int jdir, int kdir, int mode
 void launch_volume_plane(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st) {
   launch_kind<PLANE>(a, idir, jdir, kdir, mode, st);
 }
-#else
+#elif CGFD_VOLUME_KIND == 7
 void launch_volume_top(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st) {
   launch_kind<TOP>(a, idir, jdir, kdir, mode, st);
+}
+#else
+template <>
+void launch_volume_all_n<CGFD_VOLUME_KIND - 8>(const VolArgs &a, int mode, cudaStream_t st) {
+  constexpr int N = CGFD_VOLUME_KIND - 8;
+  launch_all<N / 4, N / 2 % 2, N % 2>(a, mode, st);
 }
 #endif
 

@@ -1,7 +1,9 @@
 """The volume kernels' tiles at the sizes where they change shape: interior
 boxes whose width leaves 0, 1, 8 (the most that join the x PML slab), 9 or
 31 columns beyond whole 32-point tiles, odd strike and depth sizes (a last
-block of each plane with one row at work), against the CPU oracle."""
+block of each plane with one row at work), against the CPU oracle; and the
+small grids' schedule, with the boundary kinds in one launch, against the
+separate kernels'."""
 import numpy as np
 import pytest
 
@@ -33,3 +35,46 @@ def test_leftover_columns(cgfd_lib, oracle_built, left):
         a, b = g.wavefield(c), o.wavefield(c)
         # the float32 bound of the parity tests' random-state steps
         assert np.linalg.norm(a - b) <= 2e-5 * np.linalg.norm(b), WAVE_COMPONENTS[c]
+
+
+def _cases():
+    yield "free", inputs.small_planar(nt=20)
+    yield "buried, continuity matrices", inputs.small_planar(nt=20, dynamic_method=1, free_surface=0)
+    # split nodes up to the PML: the fault planes that wait for them lie in
+    # the PML slab, edge and shell boxes too
+    yield "fault in the PML", inputs.small_planar(nt=20, margin=6)
+    yield "two faults", inputs.two_faults(nt=20)
+    p = inputs.small_planar(nt=20, ni=37, nj=59, nk=33, fault_grid=[9, 48, 9, 33], nuc_center=(27, 22))
+    yield "odd sizes", p
+
+
+@pytest.mark.parametrize("name", [n for n, _ in _cases()])
+def test_merged_boundary_launch(cgfd_lib, oracle_built, monkeypatch, name):
+    """The kinds' code is the same in both schedules: equal bit for bit, and
+    to the oracle within the rupture tests' 1e-4."""
+    p = dict(_cases())[name]
+    runs = []
+    for m in ("0", "1"):
+        monkeypatch.setenv("CGFD_MERGED", m)
+        g = Solver(p)
+        rng = np.random.default_rng(3)
+        for c in range(9):
+            g.set_wavefield(c, (rng.standard_normal((p.nk, p.nj, p.ni)) * (1e-3 if c < 3 else 1e3)).astype(np.float32))
+        g.run(9)
+        g.run_noalloc(8)
+        runs.append(g)
+    apart, together = runs
+    assert together.last_launches() < apart.last_launches()
+    o = OracleSolver(p)
+    rng = np.random.default_rng(3)
+    for c in range(9):
+        o.set_wavefield(c, (rng.standard_normal((p.nk, p.nj, p.ni)) * (1e-3 if c < 3 else 1e3)).astype(np.float32))
+    o.run(17)
+    for c in range(9):
+        a, b = apart.wavefield(c), together.wavefield(c)
+        assert np.array_equal(a, b), WAVE_COMPONENTS[c]
+        r = o.wavefield(c)
+        assert np.linalg.norm(b - r) <= 1e-4 * np.linalg.norm(r), WAVE_COMPONENTS[c]
+    for f in range(p.num_faults):
+        assert np.array_equal(apart.fault_all(f), together.fault_all(f)), f
+    assert np.array_equal(apart.stations(), together.stations())
