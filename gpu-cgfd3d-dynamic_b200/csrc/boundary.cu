@@ -78,7 +78,24 @@ __global__ void __launch_bounds__(256) k_surface_peaks(const PeakArgs a) {
     if (old[c] < val[c]) a.pg[c * n + q] = val[c];
 }
 
+// one component of a level at interior points, to or from a dense
+// [nk][nj][ni] array: a thread per point, x fastest
+template <bool GET>
+__global__ void __launch_bounds__(256) k_component(real *__restrict__ level, real *__restrict__ dense, int cmp, const Grid g) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
+  if (i >= g.ni || j >= g.nj) return;
+  const long q = i + (long)g.ni * (j + (long)g.nj * k), p = g.w(cmp, g.at(i + NG, j + NG, k + NG));
+  if (GET) dense[q] = level[p];
+  else level[p] = dense[q];
+}
+
 }  // namespace
+
+void launch_component(real *level, real *dense, int cmp, bool get, const Grid &g, cudaStream_t st) {
+  const dim3 blk(32, 8), grd((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk);
+  if (get) k_component<true><<<grd, blk, 0, st>>>(level, dense, cmp, g);
+  else k_component<false><<<grd, blk, 0, st>>>(level, dense, cmp, g);
+}
 
 int launch_sponge(const SpongeArgs &a, cudaStream_t st) {
   const long n = a.first[a.nblk];
