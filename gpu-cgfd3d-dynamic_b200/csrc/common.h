@@ -45,8 +45,9 @@ enum Met { MJAC = 0, MXIX, MXIY, MXIZ, METX, METY, METZ, MZTX, MZTY, MZTZ };
 // one medium value: (xi_x xi_y xi_z lambda), (eta_x eta_y eta_z mu),
 // (zeta_x zeta_y zeta_z 1/rho).
 #ifdef __CUDACC__
-__device__ __forceinline__ real4 coef_row(const real *cf, long scmp, int d, long q) {
-  return __ldg(reinterpret_cast<const real4 *>(cf + scmp) + d * scmp + q);
+template <class Q>
+__device__ __forceinline__ real4 coef_row(const real *cf, long scmp, int d, Q q) {
+  return __ldg((reinterpret_cast<const real4 *>(cf + scmp) + d * scmp) + q);
 }
 __device__ __forceinline__ real coef_jac(const real *cf, long q) { return __ldg(cf + q); }
 #endif
