@@ -38,6 +38,7 @@ void launch_volume_top(const VolArgs &a, int idir, int jdir, int kdir, int mode,
 int launch_fault_pre(const FaultArgs &a, const StationArgs *rec, cudaStream_t st);
 int launch_fault_post(const FaultArgs &a, cudaStream_t st);
 cudaError_t noalloc_scratch_address(real **p);
+void launch_align(const real *coef, real *coefa, long sc, cudaStream_t st);
 void launch_record(const StationArgs &a, cudaStream_t st);
 void launch_advance(Ctl *c, int max_rec, cudaStream_t st);
 void launch_fault_gather(const real *out, real *dst, int nf, const Grid &g, cudaStream_t st);
@@ -85,6 +86,7 @@ struct cgfd_solver {
   float dt = 0.f, dtmax = 0.f;
   real *w[4] = {};                      // storage slots of the 4 levels
   real *coef = nullptr, *free_mat = nullptr;    // packed metric and medium (13 scmp values)
+  real *coefa = nullptr;                // aligned grids: (xi_x eta_y lambda mu) per point
   real *abl_E = nullptr;                // sponge masks [nx | ny | nz]
   SpongeArgs sponge{};                  // sponge blocks (w set per step)
   real *pg = nullptr, *dis = nullptr;   // surface peaks [15][nj][ni], displacement [3][nj][ni]
@@ -417,7 +419,7 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
     const int sout = Lout >= 0 ? slot(Lout, it) : -1;
     VolArgs v{};
     v.g = s->g; v.cur = s->w[scur]; v.pre = s->w[spre]; v.out = sout >= 0 ? s->w[sout] : nullptr; v.end = s->w[send];
-    v.coef = s->coef; v.free_mat = s->free_mat;
+    v.coef = s->coef; v.coefa = s->coefa; v.free_mat = s->free_mat;
     v.ca = stage < 3 ? kRkA[stage] * s->dt : RL(0.0); v.cb = kRkB[stage] * s->dt; v.isfree = s->isfree;
     v.nfault = (int)s->faults.size();
     fault_planes(s, v);
@@ -772,7 +774,7 @@ static cudaError_t tune_ychunk(cgfd_solver *s) {
   const int ntiles = (key[2] + kTileY - 1) / kTileY, ip = s->it % 8, it = s->it;
   VolArgs v{};
   v.g = s->g; v.cur = s->w[slot(LP, it)]; v.pre = v.cur; v.out = s->w[slot(LA, it)]; v.end = s->w[slot(LE, it)];
-  v.coef = s->coef; v.free_mat = s->free_mat;
+  v.coef = s->coef; v.coefa = s->coefa; v.free_mat = s->free_mat;
   v.ca = kRkA[0] * s->dt; v.cb = kRkB[0] * s->dt; v.isfree = s->isfree;
   v.nfault = (int)s->faults.size();
   fault_planes(s, v);
@@ -831,6 +833,21 @@ int cgfd_upload(const cgfd_setup *su, cgfd_solver **out) {
   CK(dalloc(s, &s->free_mat, H.free_mat.size()), "free surface");
   CK(to_device(s->coef, su->coef(), su->coef_size(), s->stream), "copy metric");
   CK(to_device(s->free_mat, H.free_mat.data(), H.free_mat.size(), s->stream), "copy free");
+#ifndef CGFD_FP64
+  // aligned grids: 16 bytes more per point buy 16 bytes less in every stage
+  // and a third of the metric products.  Without the memory for it the
+  // general kernels run
+  const char *alg = std::getenv("CGFD_ALIGNED");
+  if (H.aligned && !(alg && alg[0] == '0')) {
+    if (dalloc(s, &s->coefa, 4 * (size_t)g.scmp) == cudaSuccess) {
+      launch_align(s->coef, s->coefa, g.scmp, s->stream);
+      CK(cudaGetLastError(), "aligned metric");
+    } else {
+      cudaGetLastError();
+      s->coefa = nullptr;
+    }
+  }
+#endif
   if (H.abl_nblk > 0) {
     CK(dalloc(s, &s->abl_E, (size_t)g.nx + g.ny + g.nz), "sponge");
     CK(to_device(s->abl_E, H.abl_E[0].data(), g.nx, s->stream), "copy sponge");

@@ -110,6 +110,7 @@ struct VolArgs {
   const real *cur, *pre;
   real *out, *end;            // next-stage level (null at the last stage), E
   const real *coef, *free_mat;   // packed metric and medium (coef_row / coef_jac)
+  const real *coefa;             // (xi_x eta_y lambda mu) of an aligned grid, else null
   real ca, cb;
   int isfree;
   int nfault;

@@ -248,7 +248,8 @@ int build_setup(const cgfd_config *c, HostSetup &S, std::string &msg) {
   {
     const size_t sc = g.scmp;
     float *jac = S.coef.data(), *grp = S.coef.data() + sc;
-#pragma omp parallel for schedule(static)
+    long skew = 0;
+#pragma omp parallel for schedule(static) reduction(+ : skew)
     for (int k = 0; k < nz; k++)
       for (int j = 0; j < ny; j++)
         for (int i = 0; i < nx; i++) {
@@ -260,7 +261,11 @@ int build_setup(const cgfd_config *c, HostSetup &S, std::string &msg) {
             o[0] = Mp[MXIX + 3 * r][p]; o[1] = Mp[MXIX + 3 * r + 1][p]; o[2] = Mp[MXIX + 3 * r + 2][p];
             o[3] = med[r];
           }
+          const float *x = grp + 4 * d, *y = grp + 4 * (sc + d);
+          const float ex = kAligned * std::fabs(x[0]), ey = kAligned * std::fabs(y[1]);
+          skew += !(std::fabs(x[1]) <= ex && std::fabs(x[2]) <= ex && std::fabs(y[0]) <= ey && std::fabs(y[2]) <= ey);
         }
+    S.aligned = skew == 0;
   }
 
   // ---- CFS-PML (bdry_pml_set, bdry_t.cu:80-251 and 292-440) --------------

@@ -29,6 +29,11 @@ struct FaultHost {
   std::vector<float> out;         // [11][ny*nz]
 };
 
+// An off-axis metric entry this far below its row's own is the rounding of
+// the coordinate differences that should cancel (they leave up to 2^-43 on
+// the workloads); its products are below 2^-16 of a float's last bit.
+constexpr float kAligned = 1.0f / (1ll << 40);
+
 struct HostSetup {
   Grid g;
   float dt = 0.f, dtmax = 0.f;
@@ -37,6 +42,9 @@ struct HostSetup {
   // [3][scmp][4] (metric row d, medium value d) with the medium values
   // lambda, mu, 1/rho
   std::vector<float> coef;
+  // the grid lines of x and y keep to their axis: the metric rows of x and y
+  // have one entry each, the others below kAligned of it
+  bool aligned = false;
   std::vector<float> free_mat;    // [2][ny][nx][9]: matVx2Vz, matVy2Vz at the surface
   std::vector<float> coords;      // [3][nk][nj][ni]: x, y, z of the interior grid points
   PmlHost pml[3][2];
