@@ -1458,20 +1458,17 @@ int cgfd_ensemble_run(cgfd_ensemble *e, int nsteps) {
         cgfd_solver *s = e->m[q];
         cudaStreamWaitEvent(s->stream, e->fork, 0);
         // beside the other members each member's step runs best with the y
-        // / z PML slabs on its main stream and the fault slab kernels after
-        // its interior kernel (measured: +2% over the solo default); the
+        // / z PML slabs on its main stream (six members of 2.5 M points: 3.59
+        // against 3.66 ms per step on a third stream), and its boundary kinds
+        // apart: other members fill the GPU (16 members of 0.12 M points 946
+        // against 1003 us in one launch, 12 of 0.69 M 2719 against 2982).  The
         // schedules change no arithmetic
         const int br0 = s->branches;
-        const bool pe0 = s->post_early, me0 = s->merged;
+        const bool me0 = s->merged;
         if (s->branches == 3) s->branches = 2;
-        s->post_early = false;
-        // nor do its boundary kinds share a launch: other members fill the
-        // GPU (16 members of 0.12 M points 946 against 1003 us per step, 12
-        // of 0.69 M 2719 against 2982)
         s->merged = false;
         enqueue_step(s, it, nullptr, false);
         s->branches = br0;
-        s->post_early = pe0;
         s->merged = me0;
         cudaEventRecord(e->join[q], s->stream);
         cudaStreamWaitEvent(e->origin, e->join[q], 0);
