@@ -19,16 +19,6 @@ constexpr real kB1 = RL(-7.0) / RL(6.0), kB2 = RL(8.0) / RL(6.0), kB3 = RL(-1.0)
 constexpr real kA0 = RL(1.2500392377), kA1 = RL(1.5417647610), kA2 = RL(-0.3334118088),
                kA3 = RL(0.0416862855);
 
-template <int F>
-__device__ __forceinline__ real drp(const real *__restrict__ p, long s) {
-  if (F)
-    return kC1 * __ldg(p - s) + kC2 * __ldg(p) + kC3 * __ldg(p + s) + kC4 * __ldg(p + 2 * s) + kC5 * __ldg(p + 3 * s);
-  else
-    return -(kC1 * __ldg(p + s) + kC2 * __ldg(p) + kC3 * __ldg(p - s) + kC4 * __ldg(p - 2 * s) + kC5 * __ldg(p - 3 * s));
-}
-__device__ __forceinline__ real drp_rt(const real *p, long s, int f) {
-  return f ? drp<1>(p, s) : drp<0>(p, s);
-}
 __device__ __forceinline__ real mac22(const real *p, long s, int f) {
   return f ? (__ldg(p + s) - __ldg(p)) : (__ldg(p) - __ldg(p - s));
 }
@@ -40,13 +30,6 @@ __device__ __forceinline__ real mac24(const real *p, long s, int f) {
 __device__ __forceinline__ real drp_v(const real *v, int f) {
   return f ? (kC1 * v[-1] + kC2 * v[0] + kC3 * v[1] + kC4 * v[2] + kC5 * v[3])
            : -(kC1 * v[1] + kC2 * v[0] + kC3 * v[-1] + kC4 * v[-2] + kC5 * v[-3]);
-}
-
-// offsets of the DRP stencil in table order and the matching weights
-__device__ __forceinline__ int drp_off(int f, int n) { return f ? n - 1 : n - 3; }
-__device__ __forceinline__ real drp_w(int f, int n) {
-  const real wf[5] = { kC1, kC2, kC3, kC4, kC5 };
-  return f ? wf[n] : -wf[4 - n];
 }
 
 __device__ __forceinline__ void mv3(const real *__restrict__ m, const real *v, real *o) {
