@@ -33,7 +33,10 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.join(ROOT, "gpu-cgfd3d-dynamic_b200")
 sys.path.insert(0, PKG)
 
-BYTES_PER_POINT_STEP = 624          # algorithmic HBM traffic of one point and step (FP32)
+# algorithmic HBM traffic of one point and step (FP32): 156 values, 140 where
+# the grid's x and y lines keep to their axis (all but the dipping fault)
+BYTES_PER_POINT_STEP = {"large": 624}
+BYTES_ALIGNED = 560
 FALLBACK_HBM_GBS = 6650.0
 
 
@@ -228,10 +231,10 @@ def large_case(peak, setup_free=None, warmup=3, steps=10):
     del s
     cgfd.load_library().cgfd_release_cached_memory()
     value = prob.points * steps / (run_ms / 1e3) / 1e9
-    achieved = int_pts * BYTES_PER_POINT_STEP / 4 / (int_ms / int_n / 1e3) / 1e9 if int_n else 0.0
+    achieved = int_pts * BYTES_PER_POINT_STEP["large"] / 4 / (int_ms / int_n / 1e3) / 1e9 if int_n else 0.0
     return {"workload": desc, "grid": [prob.nj, prob.ni, prob.nk], "points": prob.points, "steps": steps,
             "warmup": warmup, "value": value, "unit": "Gpt/s", "ms_per_step": run_ms / steps,
-            "interior_frac": achieved / peak, "step_frac": value * BYTES_PER_POINT_STEP / peak,
+            "interior_frac": achieved / peak, "step_frac": value * BYTES_PER_POINT_STEP["large"] / peak,
             "setup_and_upload_s": round(t_up, 1),
             "note": "device time of the same kind as value; l2: inputs larger than L2 (42 GB of wavefield levels)"}
 
@@ -357,10 +360,11 @@ def main():
     value = replicas.aggregate_rate(prob.points, args.steps, ws, run_ms_max / 1e3) / 1e9
     peak, peak_kind = peaks()
     # dominant kernel: the interior-box volume kernel; one launch is one RK
-    # stage of int_pts points at 768 / 4 = 192 algorithmic bytes each
-    bytes_per_launch = int_pts * BYTES_PER_POINT_STEP / 4
+    # stage of int_pts points at a quarter of a step's algorithmic bytes each
+    point_bytes = BYTES_PER_POINT_STEP.get(args.workload, BYTES_ALIGNED)
+    bytes_per_launch = int_pts * point_bytes / 4
     achieved = bytes_per_launch / (int_ms_max / int_n / 1e3) / 1e9 if int_n else 0.0
-    stage_bytes = vol_pts * BYTES_PER_POINT_STEP / 4
+    stage_bytes = vol_pts * point_bytes / 4
     stage_achieved = stage_bytes / (vol_ms_max / vol_n / 1e3) / 1e9
     tr = traffic_per_launch(int_pts)
     s.close()
@@ -417,8 +421,8 @@ def main():
                                           "note": "all volume kernels of one RK stage (interior, PML slabs, "
                                                   "edges and surface rows); PML auxiliary traffic is not "
                                                   "credited"},
-                         "step": {"achieved": value * 1e9 * BYTES_PER_POINT_STEP / 1e9,
-                                  "frac": value * BYTES_PER_POINT_STEP / peak}},
+                         "step": {"achieved": value * 1e9 * point_bytes / 1e9,
+                                  "frac": value * point_bytes / peak}},
             "e2e": e2e, "gpu_launches": launches, "clocks": clocks}
     if ws == 1 and args.workload == "hills" and not args.no_large:
         line["large"] = large_case(peak, setup_free=setup)

@@ -38,7 +38,7 @@ void launch_volume_top(const VolArgs &a, int idir, int jdir, int kdir, int mode,
 int launch_fault_pre(const FaultArgs &a, const StationArgs *rec, cudaStream_t st);
 int launch_fault_post(const FaultArgs &a, cudaStream_t st);
 cudaError_t noalloc_scratch_address(real **p);
-void launch_align(const real *coef, real *coefa, long sc, cudaStream_t st);
+void launch_align(const real *rows, real *out, long sc, cudaStream_t st);
 void launch_record(const StationArgs &a, cudaStream_t st);
 void launch_advance(Ctl *c, int max_rec, cudaStream_t st);
 void launch_fault_gather(const real *out, real *dst, int nf, const Grid &g, cudaStream_t st);
@@ -86,7 +86,6 @@ struct cgfd_solver {
   float dt = 0.f, dtmax = 0.f;
   real *w[4] = {};                      // storage slots of the 4 levels
   real *coef = nullptr, *free_mat = nullptr;    // packed metric and medium (13 scmp values)
-  real *coefa = nullptr;                // aligned grids: (xi_x eta_y lambda mu) per point
   real *abl_E = nullptr;                // sponge masks [nx | ny | nz]
   SpongeArgs sponge{};                  // sponge blocks (w set per step)
   real *pg = nullptr, *dis = nullptr;   // surface peaks [15][nj][ni], displacement [3][nj][ni]
@@ -145,7 +144,6 @@ struct cgfd_solver {
   // faults' 11 fields at interior nodes), a copy stream and the events that
   // order gather -> copy -> reuse (made on first use)
   real *rec_buf[2] = {};
-  real *stage = nullptr;                // one component at interior points (wavefield getter and setter)
   cudaStream_t copy = nullptr;
   cudaEvent_t ev_gathered[2] = {}, ev_copied[2] = {};
 };
@@ -419,7 +417,7 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
     const int sout = Lout >= 0 ? slot(Lout, it) : -1;
     VolArgs v{};
     v.g = s->g; v.cur = s->w[scur]; v.pre = s->w[spre]; v.out = sout >= 0 ? s->w[sout] : nullptr; v.end = s->w[send];
-    v.coef = s->coef; v.coefa = s->coefa; v.free_mat = s->free_mat;
+    v.coef = s->coef; v.free_mat = s->free_mat;
     v.ca = stage < 3 ? kRkA[stage] * s->dt : RL(0.0); v.cb = kRkB[stage] * s->dt; v.isfree = s->isfree;
     v.nfault = (int)s->faults.size();
     fault_planes(s, v);
@@ -774,7 +772,7 @@ static cudaError_t tune_ychunk(cgfd_solver *s) {
   const int ntiles = (key[2] + kTileY - 1) / kTileY, ip = s->it % 8, it = s->it;
   VolArgs v{};
   v.g = s->g; v.cur = s->w[slot(LP, it)]; v.pre = v.cur; v.out = s->w[slot(LA, it)]; v.end = s->w[slot(LE, it)];
-  v.coef = s->coef; v.coefa = s->coefa; v.free_mat = s->free_mat;
+  v.coef = s->coef; v.free_mat = s->free_mat;
   v.ca = kRkA[0] * s->dt; v.cb = kRkB[0] * s->dt; v.isfree = s->isfree;
   v.nfault = (int)s->faults.size();
   fault_planes(s, v);
@@ -825,29 +823,31 @@ int cgfd_upload(const cgfd_setup *su, cgfd_solver **out) {
   s->g = H.g; s->imethod = H.imethod; s->isfree = H.isfree; s->dt = H.dt; s->dtmax = H.dtmax;
   const char *ng = std::getenv("CGFD_NO_GRAPH");
   s->use_graph = !(ng && ng[0] == '1');
+#ifndef CGFD_FP64
+  const char *alg = std::getenv("CGFD_ALIGNED");
+  s->g.al = H.aligned && !(alg && alg[0] == '0');
+#endif
   const Grid &g = s->g;
   const size_t lev = (size_t)NCMP * g.scmp, ns = (size_t)g.ny * g.nz;
 #define CK(x, what) do { cudaError_t _e = (x); if (_e != cudaSuccess) { destroy(s); return cuda_fail(_e, what); } } while (0)
   for (int L = 0; L < 4; L++) CK(dalloc(s, &s->w[L], lev), "wavefield");
-  CK(dalloc(s, &s->coef, 13 * (size_t)g.scmp), "metric");
+  CK(dalloc(s, &s->coef, (g.al ? 9 : 13) * (size_t)g.scmp), "metric");
   CK(dalloc(s, &s->free_mat, H.free_mat.size()), "free surface");
-  CK(to_device(s->coef, su->coef(), su->coef_size(), s->stream), "copy metric");
-  CK(to_device(s->free_mat, H.free_mat.data(), H.free_mat.size(), s->stream), "copy free");
-#ifndef CGFD_FP64
-  // aligned grids: 16 bytes more per point buy 16 bytes less in every stage
-  // and a third of the metric products.  Without the memory for it the
-  // general kernels run
-  const char *alg = std::getenv("CGFD_ALIGNED");
-  if (H.aligned && !(alg && alg[0] == '0')) {
-    if (dalloc(s, &s->coefa, 4 * (size_t)g.scmp) == cudaSuccess) {
-      launch_align(s->coef, s->coefa, g.scmp, s->stream);
-      CK(cudaGetLastError(), "aligned metric");
-    } else {
-      cudaGetLastError();
-      s->coefa = nullptr;
-    }
+  if (g.al) {
+    // the Jacobian and the last group as they are; the first two are packed
+    // into one by way of a level that no step has written yet
+    const float *src = su->coef();
+    const size_t sc = g.scmp;
+    CK(to_device(s->coef, src, sc, s->stream), "copy metric");
+    CK(to_device(s->w[LA], src + sc, 8 * sc, s->stream), "copy metric");
+    CK(to_device(s->coef + 5 * sc, src + 9 * sc, 4 * sc, s->stream), "copy metric");
+    launch_align(s->w[LA], s->coef + sc, sc, s->stream);
+    CK(cudaGetLastError(), "pack metric");
+    CK(cudaMemsetAsync(s->w[LA], 0, lev * sizeof(real), s->stream), "wavefield");
+  } else {
+    CK(to_device(s->coef, su->coef(), su->coef_size(), s->stream), "copy metric");
   }
-#endif
+  CK(to_device(s->free_mat, H.free_mat.data(), H.free_mat.size(), s->stream), "copy free");
   if (H.abl_nblk > 0) {
     CK(dalloc(s, &s->abl_E, (size_t)g.nx + g.ny + g.nz), "sponge");
     CK(to_device(s->abl_E, H.abl_E[0].data(), g.nx, s->stream), "copy sponge");
@@ -1586,9 +1586,11 @@ int cgfd_get_fault_stations(cgfd_solver *s, float *out, int *nrec) {
   return get_series(s, s->fseis, s->st.nf, out, nrec);
 }
 
-// staging of one wavefield component at interior points, made on first use
-static cudaError_t stage_component(cgfd_solver *s) {
-  return s->stage ? cudaSuccess : dalloc(s, &s->stage, (size_t)s->g.ni * s->g.nj * s->g.nk);
+// A wavefield component at interior points is staged in level B, which is
+// dead between steps (every stage-2 kernel writes it before stage 3 reads it)
+// but for its ghosts, which stay zero: what was staged is cleared again.
+static cudaError_t clear_staged(cgfd_solver *s) {
+  return cudaMemsetAsync(s->w[LB], 0, (size_t)s->g.ni * s->g.nj * s->g.nk * sizeof(real), s->stream);
 }
 
 int cgfd_get_surface_peaks(cgfd_solver *s, float *out) {
@@ -1605,24 +1607,24 @@ int cgfd_get_surface_peaks(cgfd_solver *s, float *out) {
 int cgfd_get_wavefield(cgfd_solver *s, int cmp, float *out) {
   if (!s || !out || cmp < 0 || cmp >= NCMP) return fail(CGFD_ERR_ARG, "bad argument");
   const Grid &g = s->g;
-  cudaError_t e = stage_component(s);
-  if (e == cudaSuccess) {
-    launch_component(s->w[slot(LP, s->it)], s->stage, cmp, true, g, s->stream);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = to_host(out, s->stage, (size_t)g.ni * g.nj * g.nk, s->stream);
+  launch_component(s->w[slot(LP, s->it)], s->w[LB], cmp, true, g, s->stream);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = to_host(out, s->w[LB], (size_t)g.ni * g.nj * g.nk, s->stream);
+  const cudaError_t z = clear_staged(s);
+  if (e == cudaSuccess) e = z;
   return e == cudaSuccess ? CGFD_OK : cuda_fail(e, "read wavefield");
 }
 
 int cgfd_set_wavefield(cgfd_solver *s, int cmp, const float *in) {
   if (!s || !in || cmp < 0 || cmp >= NCMP) return fail(CGFD_ERR_ARG, "bad argument");
   const Grid &g = s->g;
-  cudaError_t e = stage_component(s);
-  if (e == cudaSuccess) e = to_device(s->stage, in, (size_t)g.ni * g.nj * g.nk, s->stream);
+  cudaError_t e = to_device(s->w[LB], in, (size_t)g.ni * g.nj * g.nk, s->stream);
   if (e == cudaSuccess) {
-    launch_component(s->w[slot(LP, s->it)], s->stage, cmp, false, g, s->stream);
+    launch_component(s->w[slot(LP, s->it)], s->w[LB], cmp, false, g, s->stream);
     e = cudaGetLastError();
   }
+  const cudaError_t z = clear_staged(s);
+  if (e == cudaSuccess) e = z;
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   return e == cudaSuccess ? CGFD_OK : cuda_fail(e, "write wavefield");
 }

@@ -39,19 +39,12 @@ enum Cmp { VX = 0, VY, VZ, TXX, TYY, TZZ, TYZ, TXZ, TXY };
 enum FCmp { FVX = 0, FVY, FVZ, FT2X, FT2Y, FT2Z, FT3X, FT3Y, FT3Z };
 // metric component order in the host metric block
 enum Met { MJAC = 0, MXIX, MXIY, MXIZ, METX, METY, METZ, MZTX, MZTY, MZTZ };
-// On the device the metric and the medium are one block of 13 scmp floats:
-// the Jacobian plane, then three arrays of 16-byte groups, one per
-// contravariant direction d, each holding that direction's metric row and
-// one medium value: (xi_x xi_y xi_z lambda), (eta_x eta_y eta_z mu),
-// (zeta_x zeta_y zeta_z 1/rho).
-#ifdef __CUDACC__
-template <class Q>
-__device__ __forceinline__ real4 coef_row(const real *cf, long scmp, int d, Q q) {
-  return __ldg((reinterpret_cast<const real4 *>(cf + scmp) + d * scmp) + q);
-}
-__device__ __forceinline__ real coef_jac(const real *cf, long q) { return __ldg(cf + q); }
-#endif
-
+// On the device the metric and the medium are one block: the Jacobian plane,
+// then arrays of 16-byte groups.  In general three, one per contravariant
+// direction d, each holding that direction's metric row and one medium
+// value: (xi_x xi_y xi_z lambda), (eta_x eta_y eta_z mu), (zeta_x zeta_y zeta_z
+// 1/rho).  On an aligned grid (Grid::al), whose rows of x and y have one entry
+// each, two: (xi_x eta_y lambda mu) and (zeta_x zeta_y zeta_z 1/rho).
 // per-node 3x3 fault matrices, [NFM][nodes][9]
 enum FaultMat {
   FM_D21_1 = 0, FM_D22_1, FM_D23_1, FM_D31_1, FM_D32_1, FM_D33_1,
@@ -86,6 +79,7 @@ struct Grid {
   int ni, nj, nk;        // interior points
   int nx, ny, nz;        // with ghosts
   int xoff;              // x offset of the row pitch (see above)
+  int al;                // aligned: the packed metric has two groups, not three
   long sy, sz;           // strides of j and k (elements)
   long scmp;             // elements per component (sz * nz)
   CGFD_HD long at(int i, int j, int k) const { return (long)(i + xoff) + (long)j * sy + (long)k * sz; }
@@ -94,6 +88,21 @@ struct Grid {
   // in 16-byte groups, Txy is stored alone
   CGFD_HD long w(int c, long p) const { return c < 4 ? 4 * p + c : (c < 8 ? 4 * scmp + 4 * p + (c - 4) : 8 * scmp + p); }
 };
+#ifdef __CUDACC__
+// group n of point q
+template <class Q>
+__device__ __forceinline__ real4 coef_group(const real *cf, long scmp, int n, Q q) {
+  return __ldg((reinterpret_cast<const real4 *>(cf + scmp) + n * scmp) + q);
+}
+// metric row d and medium value d of point q, whichever the grid
+__device__ __forceinline__ real4 coef_row(const Grid &g, const real *cf, int d, long q) {
+  if (!g.al) return coef_group(cf, g.scmp, d, q);
+  const real4 v = coef_group(cf, g.scmp, d == 2, q);
+  return d == 2 ? v : (d == 0 ? make_real4(v.x, 0.f, 0.f, v.z) : make_real4(0.f, v.y, 0.f, v.w));
+}
+__device__ __forceinline__ real coef_jac(const real *cf, long q) { return __ldg(cf + q); }
+#endif
+
 // distance between neighbouring points of one wavefield component (floats)
 CGFD_HD constexpr int wstep(int c) { return c < 8 ? 4 : 1; }
 

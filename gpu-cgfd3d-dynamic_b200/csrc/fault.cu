@@ -54,7 +54,7 @@ __device__ __forceinline__ void trac3(const Grid &g, const real *__restrict__ w,
                                       long q, int d, real t[3]) {
   const long sc = g.scmp;
   const real J = coef_jac(cf, q);
-  const real4 e = coef_row(cf, sc, d, q);
+  const real4 e = coef_row(g, cf, d, q);
   const real ex = e.x, ey = e.y, ez = e.z;
   // Txx ends the first 16-byte group, Tyy Tzz Tyz Txz are the second
   const real sxx = __ldg(w + g.w(TXX, q));
@@ -133,7 +133,7 @@ __device__ __forceinline__ void split_to_volume(const Grid &g, const real *__res
   real mt[3][3];   // columns e_xi, e_eta, e_zeta
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    const real4 e = coef_row(cf, sc, c, p0);
+    const real4 e = coef_row(g, cf, c, p0);
     mt[0][c] = e.x; mt[1][c] = e.y; mt[2][c] = e.z;
   }
   const real rj = 1.0f / coef_jac(cf, p0);
@@ -245,7 +245,7 @@ __device__ __forceinline__ bool slab_item(const FaultArgs &a, long t, int &j, in
 __device__ __forceinline__ void slab_velocity(const FaultArgs &a, int j, int k, int s, real hv3[3]) {
   const Grid &g = a.g;
   const int J = j + NG, K = k + NG;
-  const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny, sc = g.scmp;
+  const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny;
   const FaultDev &F = a.F;
   const int i0 = F.i0;
   const int km = g.nk - (k + 1);
@@ -288,7 +288,7 @@ __device__ __forceinline__ void slab_velocity(const FaultArgs &a, int j, int k, 
 
   // y and z lines of T2 = J e_eta . sigma and T3 = J e_zeta . sigma
   const real *t2 = tr + 3 * pl + trac_slot(s), *t3 = t2 + 3 * pl;
-  const real rr = coef_row(a.coef, sc, 2, q).w / coef_jac(a.coef, q);
+  const real rr = coef_row(g, a.coef, 2, q).w / coef_jac(a.coef, q);
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     real y[7], z[7];
@@ -345,7 +345,7 @@ __device__ __forceinline__ void vel_mac22(const real4 *__restrict__ p, long st, 
 __device__ __forceinline__ void slab_stress(const FaultArgs &a, int j, int k, int s, real h[6]) {
   const Grid &g = a.g;
   const int J = j + NG, K = k + NG;
-  const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny, sc = g.scmp;
+  const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny;
   const int i0 = a.F.i0;
   const real *w = a.wcur;
   const int km = g.nk - (k + 1);
@@ -410,7 +410,7 @@ __device__ __forceinline__ void slab_stress(const FaultArgs &a, int j, int k, in
 #pragma unroll
     for (int c = 0; c < 3; c++) dz[c] = o1[c] + o2[c];
   }
-  const real4 r0 = coef_row(a.coef, sc, 0, q), r1 = coef_row(a.coef, sc, 1, q), r2 = coef_row(a.coef, sc, 2, q);
+  const real4 r0 = coef_row(g, a.coef, 0, q), r1 = coef_row(g, a.coef, 1, q), r2 = coef_row(g, a.coef, 2, q);
   const real e[3][3] = { { r0.x, r0.y, r0.z }, { r1.x, r1.y, r1.z }, { r2.x, r2.y, r2.z } };
   const real lam = r0.w, mu = r1.w;
   const real l2m = lam + 2.0f * mu;
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(192) k_fault_split(const FaultArgs a) {
   const int tx = threadIdx.x, q = threadIdx.y, m = q / 3, c = q - 3 * m;
   const int j = a.j0 + blockIdx.x * 32 + tx, k = a.k0 + blockIdx.y;
   const int J = j + NG, K = k + NG;
-  const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny, ny = g.ny, sc = g.scmp;
+  const long ns = (long)g.ny * g.nz, nd = J + (long)K * g.ny, ny = g.ny;
   const uint8_t fl = j < a.j0 + a.nj ? F.flag[nd] : 0;
   const bool act = fl & FL_SPLIT;
   const int i0 = F.i0, mode = a.mode;
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(192) k_fault_split(const FaultArgs a) {
   if (act) {
     // what the friction law reads of this node
     jac0 = coef_jac(cf, p0);
-    exi = coef_row(cf, sc, 0, p0);
+    exi = coef_row(g, cf, 0, p0);
     rho0 = F.scal[FS_RHO0 * ns + nd]; rho1 = F.scal[FS_RHO1 * ns + nd];
     slip = F.out[CGFD_FAULT_SLIP * ns + nd];
     mus = F.scal[FS_MUS * ns + nd]; mud = F.scal[FS_MUD * ns + nd];

@@ -92,8 +92,7 @@ struct VolArgs {
   VolBox box[kMaxBoxes];
   const real *cur, *pre;
   real *out, *end;            // next-stage level (null at the last stage), E
-  const real *coef, *free_mat;   // packed metric and medium (coef_row / coef_jac)
-  const real *coefa;             // (xi_x eta_y lambda mu) of an aligned grid, else null
+  const real *coef, *free_mat;   // packed metric and medium (coef_group, coef_row, coef_jac)
   real ca, cb;
   int isfree;
   int nfault;
@@ -119,7 +118,7 @@ struct FaultArgs {
   FaultDev F;
   const real *wcur, *wpre;
   real *wout, *wend;
-  const real *coef, *free_mat;   // packed metric and medium (coef_row / coef_jac)
+  const real *coef, *free_mat;   // packed metric and medium (coef_group, coef_row, coef_jac)
   // fault wavefield levels [9][2 sides][ny*nz]: stage input, time-n level,
   // next-stage output (null at the last stage), fourth level (V, then n+1)
   const real *fc, *fp;

@@ -125,6 +125,7 @@ int build_setup(const cgfd_config *c, HostSetup &S, std::string &msg) {
     // 8 points of 16-byte groups per 128-byte line (the double build's
     // 32-byte groups need a multiple of 4, which this also is)
     g.xoff = (8 - (ilo + NG) % 8) % 8;
+    g.al = 0;   // set when a solver is made
   }
   g.sy = ((g.nx + g.xoff + 31) / 32) * 32;
   g.sz = g.sy * g.ny;

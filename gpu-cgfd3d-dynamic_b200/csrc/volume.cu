@@ -45,19 +45,26 @@ namespace {
 
 constexpr int BX = kTileX, BY = kTileY;
 
-// conservative traction J * (e . sigma_row) at point q for metric row d
+// conservative traction J * (e . sigma_row) at point q for metric row DIR
 // (0: xi, 1: eta, 2: zeta), all three stress rows (xx,xy,xz), (xy,yy,yz),
 // (xz,yz,zz)
+template <int DIR, bool AL>
 __device__ __forceinline__ void ctrac3(const Grid &g, const real *__restrict__ w, const real *__restrict__ cf,
-                                       long q, int d, real t[3]) {
-  const real4 e = coef_row(cf, g.scmp, d, q);
+                                       long q, real t[3]) {
+  const real4 e = coef_group(cf, g.scmp, AL ? DIR / 2 : DIR, q);
   const real J = coef_jac(cf, q);
   const real sxx = __ldg(w + g.w(TXX, q)), sxy = __ldg(w + g.w(TXY, q));
   const real4 s4 = __ldg(reinterpret_cast<const real4 *>(w + 4 * g.scmp) + q);   // Tyy Tzz Tyz Txz
   const real syy = s4.x, szz = s4.y, syz = s4.z, sxz = s4.w;
-  t[0] = J * (e.x * sxx + e.y * sxy + e.z * sxz);
-  t[1] = J * (e.x * sxy + e.y * syy + e.z * syz);
-  t[2] = J * (e.x * sxz + e.y * syz + e.z * szz);
+  if (AL && DIR == 0) {
+    t[0] = J * (e.x * sxx); t[1] = J * (e.x * sxy); t[2] = J * (e.x * sxz);
+  } else if (AL && DIR == 1) {
+    t[0] = J * (e.y * sxy); t[1] = J * (e.y * syy); t[2] = J * (e.y * syz);
+  } else {
+    t[0] = J * (e.x * sxx + e.y * sxy + e.z * sxz);
+    t[1] = J * (e.x * sxy + e.y * syy + e.z * syz);
+    t[2] = J * (e.x * sxz + e.y * syz + e.z * szz);
+  }
 }
 
 // The point's three groups within one level: pointers to the point itself,
@@ -496,11 +503,8 @@ __device__ __forceinline__ void volume_point(const VolArgs &a, int i, int j, int
     if (kn < g.nz) prefetch9(a.cur, sc, p + (kn - K) * sz);
     if (kc < g.nz) {
 #pragma unroll
-      for (int d = AL ? 1 : 0; d < 3; d++) {
-        const real4 *c = AL && d == 1 ? reinterpret_cast<const real4 *>(a.coefa)
-                                      : reinterpret_cast<const real4 *>(a.coef + sc + 4 * d * sc);
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(c + (p + CGFD_AHEAD * sz)));
-      }
+      for (int n = 0; n < (AL ? 2 : 3); n++)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const real4 *>(a.coef + sc + 4 * n * sc) + (p + CGFD_AHEAD * sz)));
     }
   }
 #endif
@@ -517,13 +521,11 @@ __device__ __forceinline__ void volume_point(const VolArgs &a, int i, int j, int
   const V9 c0 = tap9<true>(w, 0);
   real v0[9];
   unpack9(c0, v0);
-  // the metric rows and the medium; an aligned grid has (xi_x eta_y lambda
-  // mu) in one group
-  const real4 zero = make_real4(0.f, 0.f, 0.f, 0.f);
-  const real4 al = AL ? __ldg(reinterpret_cast<const real4 *>(a.coefa) + p) : zero;
-  const real4 r0 = AL ? make_real4(al.x, 0.f, 0.f, al.z) : coef_row(a.coef, sc, 0, p);
-  const real4 r1 = AL ? make_real4(0.f, al.y, 0.f, al.w) : coef_row(a.coef, sc, 1, p);
-  const real4 r2 = coef_row(a.coef, sc, 2, p);
+  // the metric rows and the medium
+  const real4 g0 = coef_group(a.coef, sc, 0, p), g1 = coef_group(a.coef, sc, 1, p);
+  const real4 r0 = AL ? make_real4(g0.x, 0.f, 0.f, g0.z) : g0;
+  const real4 r1 = AL ? make_real4(0.f, g0.y, 0.f, g0.w) : g1;
+  const real4 r2 = AL ? g1 : coef_group(a.coef, sc, 2, p);
   const real e[3][3] = { { r0.x, r0.y, r0.z }, { r1.x, r1.y, r1.z }, { r2.x, r2.y, r2.z } };
   const real lam = r0.w, mu = r1.w, slw = r2.w;
   const real l2m = lam + 2.0f * mu;
@@ -645,13 +647,13 @@ __device__ __forceinline__ void volume_point(const VolArgs &a, int i, int j, int
     real t[3];
 #pragma unroll
     for (int n = 0; n < 5; n++) {
-      ctrac3(g, cur, a.coef, p + (ID ? n - 1 : n - 3), 0, t);
+      ctrac3<0, AL>(g, cur, a.coef, p + (ID ? n - 1 : n - 3), t);
 #pragma unroll
       for (int rr = 0; rr < 3; rr++) dx[rr] += wdrp<ID>(n) * t[rr];
     }
 #pragma unroll
     for (int n = 0; n < 5; n++) {
-      ctrac3(g, cur, a.coef, p + (JD ? n - 1 : n - 3) * sy, 1, t);
+      ctrac3<1, AL>(g, cur, a.coef, p + (JD ? n - 1 : n - 3) * sy, t);
 #pragma unroll
       for (int rr = 0; rr < 3; rr++) dy[rr] += wdrp<JD>(n) * t[rr];
     }
@@ -661,7 +663,7 @@ __device__ __forceinline__ void volume_point(const VolArgs &a, int i, int j, int
       if (kk == nk2) {
         t[0] = t[1] = t[2] = 0.f;
       } else {
-        ctrac3(g, cur, a.coef, g.at(I, J, kk < nk2 ? kk : 2 * nk2 - kk), 2, t);
+        ctrac3<2, AL>(g, cur, a.coef, g.at(I, J, kk < nk2 ? kk : 2 * nk2 - kk), t);
         if (kk > nk2) { t[0] = -t[0]; t[1] = -t[1]; t[2] = -t[2]; }
       }
 #pragma unroll
@@ -754,7 +756,7 @@ void launch_dirs(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaS
 template <int KIND>
 void launch_kind(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st) {
 #ifndef CGFD_FP64
-  if (a.coefa) return launch_dirs<KIND, true>(a, idir, jdir, kdir, mode, st);
+  if (a.g.al) return launch_dirs<KIND, true>(a, idir, jdir, kdir, mode, st);
 #endif
   launch_dirs<KIND, false>(a, idir, jdir, kdir, mode, st);
 }
@@ -814,15 +816,16 @@ void launch_volume_all(const VolArgs &a, int idir, int jdir, int kdir, int mode,
 void launch_volume_interior(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st) {
   launch_kind<INTERIOR>(a, idir, jdir, kdir, mode, st);
 }
-// (xi_x eta_y lambda mu) of every point of an aligned grid
-__global__ void __launch_bounds__(256) k_align(const real *__restrict__ coef, real *__restrict__ coefa, long sc) {
+// the first group of an aligned grid, (xi_x eta_y lambda mu), of every point
+// from the general rows 0 and 1
+__global__ void __launch_bounds__(256) k_align(const real4 *__restrict__ rows, real4 *__restrict__ out, long sc) {
   const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= sc) return;
-  const real4 r0 = coef_row(coef, sc, 0, p), r1 = coef_row(coef, sc, 1, p);
-  reinterpret_cast<real4 *>(coefa)[p] = make_real4(r0.x, r1.y, r0.w, r1.w);
+  const real4 r0 = rows[p], r1 = rows[sc + p];
+  out[p] = make_real4(r0.x, r1.y, r0.w, r1.w);
 }
-void launch_align(const real *coef, real *coefa, long sc, cudaStream_t st) {
-  k_align<<<(unsigned)((sc + 255) / 256), 256, 0, st>>>(coef, coefa, sc);
+void launch_align(const real *rows, real *out, long sc, cudaStream_t st) {
+  k_align<<<(unsigned)((sc + 255) / 256), 256, 0, st>>>(reinterpret_cast<const real4 *>(rows), reinterpret_cast<real4 *>(out), sc);
 }
 #elif CGFD_VOLUME_KIND == 1
 void launch_volume_shell(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st) {
@@ -857,7 +860,7 @@ template <>
 void launch_volume_all_n<CGFD_VOLUME_KIND - 8>(const VolArgs &a, int mode, cudaStream_t st) {
   constexpr int N = CGFD_VOLUME_KIND - 8;
 #ifndef CGFD_FP64
-  if (a.coefa) return launch_all<N / 4, N / 2 % 2, N % 2, true>(a, mode, st);
+  if (a.g.al) return launch_all<N / 4, N / 2 % 2, N % 2, true>(a, mode, st);
 #endif
   launch_all<N / 4, N / 2 % 2, N % 2, false>(a, mode, st);
 }

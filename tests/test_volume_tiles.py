@@ -108,3 +108,26 @@ def test_aligned_grid_kernels(cgfd_lib, oracle_built, monkeypatch, name):
         assert np.linalg.norm(a - b) <= 1e-6 * np.linalg.norm(a), WAVE_COMPONENTS[c]
     # rounding differs where the aligned kernels ran, and only there
     assert same == (name == "sheared")
+
+
+@pytest.mark.parametrize("pml", [0, 5])
+def test_getter_and_setter_leave_the_step_alone(cgfd_lib, pml):
+    """Wavefield reads and writes stage a component in a level that is dead
+    between steps; its ghost points, which taps at the grid's sides read, must
+    be zero again afterwards.  37x59x33 points: rows that fill no tile."""
+    p = inputs.small_planar(nt=20, ni=37, nj=59, nk=33, fault_grid=[9, 48, 9, 33], nuc_center=(27, 22), pml=pml)
+    rng = np.random.default_rng(1)
+    f = [(rng.standard_normal((p.nk, p.nj, p.ni)) * (1e-3 if c < 3 else 1e3)).astype(np.float32) for c in range(9)]
+    g, h = Solver(p), Solver(p)
+    for s in (g, h):
+        for c in range(9):
+            s.set_wavefield(c, f[c])
+    for c in range(9):
+        assert np.array_equal(g.wavefield(c), f[c]), WAVE_COMPONENTS[c]
+    g.run(8)
+    for _ in range(8):
+        h.run(1)
+        for c in (0, 8):
+            h.set_wavefield(c, h.wavefield(c))
+    for c in range(9):
+        assert np.array_equal(g.wavefield(c), h.wavefield(c)), WAVE_COMPONENTS[c]
