@@ -17,8 +17,8 @@ LIB = os.path.join(LIBDIR, "libcgfd.so")
 # the same kernels computing in double (-DCGFD_FP64), for error statements
 # of the float build against a double build on the same inputs
 LIB64 = os.path.join(LIBDIR, "libcgfd64.so")
-# the volume kernels' hundreds of instantiations compress to a tenth
-ARCH = ["-gencode", "arch=compute_100a,code=sm_100a", "--compress-mode=size"]
+# the volume kernels have hundreds of instantiations; compressed to a third
+ARCH = ["-gencode", "arch=compute_100a,code=sm_100a", "-Xfatbin=-compress-all"]
 NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 
 # (source, object, extra flags): the volume kernels build as one unit per
