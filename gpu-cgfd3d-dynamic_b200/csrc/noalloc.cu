@@ -2,7 +2,7 @@
 //
 // cgfd_run_noalloc advances a solver without allocating anything.  The one
 // buffer a time step needs beyond the solver's own state is the per-stage
-// traction scratch of the fault kernels (k_fault_trac writes it, the trial
+// traction scratch of the fault kernels (k_fault_pre writes it, the trial
 // and slab-velocity kernels read it).  cgfd_run keeps a scratch allocated
 // with the solver; the no-alloc entry point uses this file-scope device
 // array instead.  Its size is fixed at build time (CGFD_NOALLOC_SCRATCH_FLOATS

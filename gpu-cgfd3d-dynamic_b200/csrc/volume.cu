@@ -20,7 +20,8 @@
 // and the bottom ring run k_volume<EDGE>; the four rows under the free
 // surface run k_volume<TOP> away from the PML columns and k_volume<SHELL>
 // in them; the fault planes' welded points next to split nodes run
-// k_volume<PLANE> after the first fault kernels.  Each stage reads the
+// k_volume<PLANE> after the first fault kernels.  On small grids
+// k_volume_all runs all boundary boxes in one launch.  Each stage reads the
 // input level (stencil taps come from L1/L2), the metric and the medium
 // once and writes the output levels once; each thread asks L2 early for
 // the lines it reads last (prefetch), and interior threads for the next z
@@ -28,13 +29,15 @@
 //
 // A level stores the nine components of a point in two 16-byte groups and
 // one real (Grid::w), so a stencil tap is three loads: x taps are
-// immediate offsets from three base pointers, y / z taps share two int
-// offset tables, the centre sample is loaded once for all three
+// immediate offsets from the point's three pointers, y / z taps share two
+// int offset tables, the centre sample is loaded once for all three
 // directions.  The RHS is built direction by direction, so a PML face of
 // normal d reuses direction d's contribution.
 //
-// Roofline: HBM-bound.  Algorithmic traffic per point and step is
-// 156 floats = 624 B (21+9, 30+18, 30+9, 30+9 floats over the 4 stages).
+// Roofline: algorithmic traffic per point and step is 156 floats = 624 B
+// (21+9, 30+18, 30+9, 30+9 floats over the 4 stages), 140 on aligned grids.
+// In practice large grids also meet the 1000 W limit and the interior kernel
+// the L1 data pipe (13 taps of 36 bytes a point), small ones latency.
 #include <cuda_runtime.h>
 
 #include "ops.cuh"
