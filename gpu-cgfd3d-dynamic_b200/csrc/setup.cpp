@@ -262,6 +262,8 @@ int build_setup(const cgfd_config *c, HostSetup &S, std::string &msg) {
             o[0] = Mp[MXIX + 3 * r][p]; o[1] = Mp[MXIX + 3 * r + 1][p]; o[2] = Mp[MXIX + 3 * r + 2][p];
             o[3] = med[r];
           }
+          // (the ghosts' metric only ever multiplies stresses that are zero)
+          if (i < ni1 || i > ni2 || j < nj1 || j > nj2 || k < nk1 || k > nk2) continue;
           const float *x = grp + 4 * d, *y = grp + 4 * (sc + d);
           const float ex = kAligned * std::fabs(x[0]), ey = kAligned * std::fabs(y[1]);
           skew += !(std::fabs(x[1]) <= ex && std::fabs(x[2]) <= ex && std::fabs(y[0]) <= ey && std::fabs(y[2]) <= ey);
