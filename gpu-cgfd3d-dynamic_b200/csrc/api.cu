@@ -1443,7 +1443,14 @@ int cgfd_ensemble_run(cgfd_ensemble *e, int nsteps) {
   const int n = (int)e->m.size();
   for (int q = 1; q < n; q++)
     if (e->m[q]->it != e->m[0]->it) return fail(CGFD_ERR_STATE, "ensemble members out of step (cgfd_run on a member?)");
-  cudaError_t er;
+  cudaError_t er = cudaSuccess;
+  // the graphs run on the ensemble's own stream: what the members' calls have
+  // left on theirs (the clear after a wavefield read) comes first
+  for (int q = 0; q < n && er == cudaSuccess; q++) {
+    er = cudaEventRecord(e->join[q], e->m[q]->stream);
+    if (er == cudaSuccess) er = cudaStreamWaitEvent(e->origin, e->join[q], 0);
+  }
+  if (er != cudaSuccess) return cuda_fail(er, "ensemble members' streams");
   for (int step = 0; step < nsteps; step++) {
     const int it = e->m[0]->it;
     cudaGraphExec_t &G = e->graph[it % 8];
@@ -1588,7 +1595,9 @@ int cgfd_get_fault_stations(cgfd_solver *s, float *out, int *nrec) {
 
 // A wavefield component at interior points is staged in level B, which is
 // dead between steps (every stage-2 kernel writes it before stage 3 reads it)
-// but for its ghosts, which stay zero: what was staged is cleared again.
+// but for its ghosts, which stay zero: what was staged is cleared again.  The
+// getter does not wait for the clear: the solver's steps follow it on its
+// stream, an ensemble's graphs wait for their members' streams.
 static cudaError_t clear_staged(cgfd_solver *s) {
   return cudaMemsetAsync(s->w[LB], 0, (size_t)s->g.ni * s->g.nj * s->g.nk * sizeof(real), s->stream);
 }
