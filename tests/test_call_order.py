@@ -7,6 +7,7 @@ the GPU: the same call sequences against their plain counterparts."""
 import ctypes
 import glob
 import os
+import re
 import subprocess
 
 import numpy as np
@@ -68,6 +69,23 @@ def unordered_before_graphs(ops):
     return found
 
 
+def kernel(name):
+    """Short name of a launched kernel; k_volume with its kind."""
+    kind = re.search(r"k_volumeI(?:Li\dE){4}Li(\d)E", name)
+    return f"k_volume {kind.group(1)}" if kind else re.search(r"k_(?:fault_)?[a-z]+(?:_[a-z]+)?", name).group(0)
+
+
+def clear_of_the_pml(nt=20):
+    """A fault whose neighbourhood (i0 +- 6, split box + 3 nodes) stays clear of
+    every PML slab and edge box, as on the large workloads, on a grid small
+    enough that the boundary kinds run in one launch by default."""
+    p = inputs.tpv_planar(ni=40, nj=80, nk=40, fault_x_index=21, fault_grid=[25, 56, 15, 40], nuc_half=3,
+                          pml=5, nt=nt, nsta=4, margin=10)
+    i0 = p.fault_x_index[0] - 1
+    assert i0 - 6 > 5 and i0 + 6 < p.ni - 6 and p.welded_margin - 3 > 5
+    return p
+
+
 def closed_box(**kw):
     """A small rupture without a free surface (whose steps the recording
     runtime counts)."""
@@ -110,3 +128,58 @@ def test_ensemble_after_a_wavefield_read(cgfd_lib):
             assert np.array_equal(s.wavefield(c), m.wavefield(c)), c
         assert np.array_equal(s.fault_all(), m.fault_all())
     ens.close()
+
+
+def test_which_schedule_a_switch_gives(recording, monkeypatch):
+    """Without the one boundary launch of small grids the next stage's first
+    fault kernels are issued before a stage's PML kernels (what every large
+    grid does), with CGFD_PRE_EARLY=0 after them."""
+    from cgfd import Solver
+    p = clear_of_the_pml()
+
+    def step(**env):
+        for k, v in env.items():
+            monkeypatch.setenv(k, v)
+        s = Solver(p, lib=recording)
+        for k in env:
+            monkeypatch.delenv(k)
+        ops = operations(recording)
+        s.close()
+        first = next(n for n, o in enumerate(ops) if o[0] == "begin")
+        last = next(n for n, o in enumerate(ops) if o[0] == "end")
+        return [(kernel(o[2]), o[1]) for o in ops[first:last] if o[0] == "launch"]
+
+    assert any(k == "k_volume_all" for k, _ in step())
+    for env, early in (({"CGFD_MERGED": "0"}, True), ({"CGFD_PRE_EARLY": "0"}, False)):
+        launches = step(**env)
+        names = [k for k, _ in launches]
+        assert "k_volume_all" not in names
+        pre = [n for n, k in enumerate(names) if k == "k_fault_pre"]
+        face_x = [n for n, k in enumerate(names) if k == "k_volume 2"]
+        assert len(pre) == len(face_x) == 4
+        assert [pre[n + 1] < face_x[n] for n in range(3)] == [early] * 3
+        # three branches, the fault's on a stream of its own
+        assert len({st for _, st in launches}) == 3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("serial", [("CGFD_PRE_EARLY", "0"), ("CGFD_BRANCHES", "0")])
+def test_early_schedule_is_the_serial_one_bit_for_bit(cgfd_lib, monkeypatch, serial):
+    """The schedule that large grids run (three branches, the fault kernels
+    beside the interior and ahead of the PML kernels, the slabs right after
+    them), here with CGFD_MERGED=0, against the same kernels one after the
+    other."""
+    from cgfd import Solver, WAVE_COMPONENTS
+    p = clear_of_the_pml(nt=60)
+    monkeypatch.setenv("CGFD_MERGED", "0")
+    early = Solver(p)
+    monkeypatch.setenv(*serial)
+    other = Solver(p)
+    for s in (early, other):
+        s.run(60)
+    assert early.fault("Vs").max() > 0.1
+    for f in ("Vs", "Slip", "Tn", "Ts1"):
+        assert np.array_equal(early.fault(f), other.fault(f)), f
+    for c in WAVE_COMPONENTS:
+        assert np.array_equal(early.wavefield(c), other.wavefield(c)), c
+    assert np.array_equal(early.stations(), other.stations())
