@@ -131,7 +131,8 @@ struct cgfd_solver {
   long long vol_launches = 0, int_launches = 0;
   long long int_points = 0, vol_points = 0;   // points one launch updates
   int it = 0;
-  long long launches_per_step = 0, last_launches = 0;
+  long long graph_launches[2][8] = {};  // kernels in each graph
+  long long last_launches = 0;
   int ychunk = 16;                      // interior kernel: y tiles per z-marching chunk (set at upload)
   bool pack = true;                     // pack boxes at most 24 points wide (x PML slabs)
   // boxes of each volume kernel kind: 0 interior, 1 generic shell (PML
@@ -277,7 +278,7 @@ size_t trac_slices(const cgfd_solver *s, size_t *off) {
 // traction scratch to use instead of each fault's own (cgfd_run_noalloc),
 // split into one slice per fault because the first fault kernels of every
 // fault run before the later ones of any fault; timed: whether the
-// solver's timing events may be recorded
+// solver's timing events may be recorded; returns the number of launches
 // the fault planes of a volume launch: x = i0 of each fault, its split-node
 // flags and the deferred box (the split box grown by 3 nodes, empty when the
 // fault has no split node)
@@ -334,7 +335,7 @@ bool late_boxes(const cgfd_solver *s, VolArgs &v) {
   return ok;
 }
 
-void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = true) {
+long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = true) {
   const int ip = it % 8;
   const bool tm = s->timing && timed;
   long long nl = 0;
@@ -628,7 +629,7 @@ void enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = tru
     launch_advance(s->ctl, s->st.max_rec, s->stream);
     nl++;
   }
-  s->launches_per_step = nl;
+  return nl;
 }
 
 int cuda_fail(cudaError_t e, const char *what) {
@@ -1142,7 +1143,7 @@ static int build_graph(cgfd_solver *s, int it) {
   cudaGraph_t gr;
   cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(e, "begin capture");
-  enqueue_step(s, it);
+  s->graph_launches[s->timing][it % 8] = enqueue_step(s, it);
   // a launch refused during capture (bad configuration) is not part of the
   // graph and would otherwise go unnoticed
   const cudaError_t le = cudaGetLastError();
@@ -1213,12 +1214,12 @@ int cgfd_run(cgfd_solver *s, int nsteps) {
       }
       e = cudaGraphLaunch(G, s->stream);
       if (e != cudaSuccess) return cuda_fail(e, "graph launch");
+      nl += s->graph_launches[s->timing][it % 8];
     } else {
-      enqueue_step(s, it);
+      nl += enqueue_step(s, it);
       e = cudaGetLastError();
       if (e != cudaSuccess) return cuda_fail(e, "launch");
     }
-    nl += s->launches_per_step;
     s->it++;
   }
   e = cudaEventRecord(s->ev_run[1], s->stream);
@@ -1300,11 +1301,11 @@ int cgfd_run_fault_output(cgfd_solver *s, int nsteps, int every, float *out, lon
         if (rc != CGFD_OK) return rc;
       }
       e = cudaGraphLaunch(G, s->stream);
+      nl += s->graph_launches[s->timing][it % 8];
     } else {
-      enqueue_step(s, it);
+      nl += enqueue_step(s, it);
       e = cudaGetLastError();
     }
-    nl += s->launches_per_step;
     s->it++;
   }
   if (e == cudaSuccess) e = cudaEventRecord(s->ev_run[1], s->stream);
@@ -1383,10 +1384,9 @@ int cgfd_run_noalloc(cgfd_solver *s, int nsteps) {
   s->run_ms = s->vol_ms = s->int_ms = 0;
   s->vol_launches = s->int_launches = 0;
   for (int q = 0; q < nsteps; q++) {
-    enqueue_step(s, s->it, trac, false);
+    nl += enqueue_step(s, s->it, trac, false);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail_fixed_cuda(e, "cgfd_run_noalloc: launch");
-    nl += s->launches_per_step;
     s->it++;
   }
   s->last_launches = nl;
@@ -1407,6 +1407,7 @@ struct cgfd_ensemble {
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> join;
   cudaGraphExec_t graph[8] = {};
+  std::vector<long long> launches[8];   // each member's kernels in each graph
 };
 
 static void ensemble_free(cgfd_ensemble *e) {
@@ -1451,6 +1452,7 @@ int cgfd_ensemble_run(cgfd_ensemble *e, int nsteps) {
     if (er == cudaSuccess) er = cudaStreamWaitEvent(e->origin, e->join[q], 0);
   }
   if (er != cudaSuccess) return cuda_fail(er, "ensemble members' streams");
+  std::vector<long long> ran(n, 0);
   for (int step = 0; step < nsteps; step++) {
     const int it = e->m[0]->it;
     cudaGraphExec_t &G = e->graph[it % 8];
@@ -1461,6 +1463,7 @@ int cgfd_ensemble_run(cgfd_ensemble *e, int nsteps) {
       er = cudaStreamBeginCapture(e->origin, cudaStreamCaptureModeThreadLocal);
       if (er != cudaSuccess) return cuda_fail(er, "begin ensemble capture");
       cudaEventRecord(e->fork, e->origin);
+      e->launches[it % 8].assign(n, 0);
       for (int q = 0; q < n; q++) {
         cgfd_solver *s = e->m[q];
         cudaStreamWaitEvent(s->stream, e->fork, 0);
@@ -1474,7 +1477,7 @@ int cgfd_ensemble_run(cgfd_ensemble *e, int nsteps) {
         const bool me0 = s->merged;
         if (s->branches == 3) s->branches = 2;
         s->merged = false;
-        enqueue_step(s, it, nullptr, false);
+        e->launches[it % 8][q] = enqueue_step(s, it, nullptr, false);
         s->branches = br0;
         s->merged = me0;
         cudaEventRecord(e->join[q], s->stream);
@@ -1493,13 +1496,16 @@ int cgfd_ensemble_run(cgfd_ensemble *e, int nsteps) {
     }
     er = cudaGraphLaunch(G, e->origin);
     if (er != cudaSuccess) return cuda_fail(er, "ensemble graph launch");
-    for (cgfd_solver *s : e->m) { s->it++; s->last_launches = 0; }
+    for (int q = 0; q < n; q++) {
+      e->m[q]->it++;
+      ran[q] += e->launches[it % 8][q];
+    }
   }
   er = cudaStreamSynchronize(e->origin);
   if (er != cudaSuccess) return cuda_fail(er, "ensemble run");
+  for (int q = 0; q < n; q++) e->m[q]->last_launches = ran[q];
   for (int q = 0; q < n; q++) {
     cgfd_solver *s = e->m[q];
-    s->last_launches = (long long)nsteps * s->launches_per_step;
     Ctl c;
     er = cudaMemcpy(&c, s->ctl, sizeof c, cudaMemcpyDeviceToHost);
     if (er != cudaSuccess) return cuda_fail(er, "read control block");

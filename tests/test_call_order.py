@@ -183,3 +183,50 @@ def test_early_schedule_is_the_serial_one_bit_for_bit(cgfd_lib, monkeypatch, ser
     for c in WAVE_COMPONENTS:
         assert np.array_equal(early.wavefield(c), other.wavefield(c)), c
     assert np.array_equal(early.stations(), other.stations())
+
+
+def test_launch_counts_are_those_of_the_schedule_that_ran(recording, monkeypatch):
+    """last_launches is the count of the graph that ran, whatever other
+    schedule of the solver was enqueued last: timed graphs, an ensemble's,
+    direct launches."""
+    import cgfd
+    monkeypatch.setattr(cgfd, "load_library", lambda *a: recording)
+    a, b = (cgfd.Solver(closed_box(seed=q), lib=recording) for q in (7, 8))
+    kernels, inside = {}, None       # kernels of each captured graph
+
+    def launched():
+        """Kernels launched since the last look, directly or in graphs."""
+        nonlocal inside
+        n = 0
+        for op, st, *rest in operations(recording):
+            if op == "begin":
+                inside = 0
+            elif op == "end":
+                kernels[rest[0]], inside = inside, None
+            elif op == "launch" and inside is not None:
+                inside += 1
+            elif op == "launch":
+                n += 1
+            elif op == "graph":
+                n += kernels[rest[0]]
+        return n
+
+    launched()
+    ens = cgfd.Ensemble([a, b])
+
+    def check(call, solvers):
+        call()
+        assert sum(s.last_launches() for s in solvers) == launched()
+
+    for timing in (False, True, False):
+        a.set_timing(timing)
+        b.set_timing(timing)
+        launched()
+        check(lambda: a.run(3), [a])
+        check(lambda: b.run(3), [b])
+        check(lambda: ens.run(2), [a, b])
+        check(lambda: a.run(1), [a])
+        check(lambda: b.run_noalloc(1), [b])
+        check(lambda: a.run(9), [a])
+        check(lambda: b.run(9), [b])
+    ens.close()
