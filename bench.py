@@ -416,6 +416,8 @@ def main():
                          "peak_source": peak_kind, "traffic": tr, "algorithmic_bytes_per_launch": bytes_per_launch,
                          "points_per_launch": int_pts, "launch_ms": int_ms_max / max(int_n, 1),
                          "interior_share_of_step": int_ms_max / run_ms_max,
+                         "launch_note": "start to end of the launch; the fault kernels, and on grids of a few "
+                                        "million points or less the boundary kinds, run beside it",
                          "volume_stage": {"achieved": stage_achieved, "frac": stage_achieved / peak,
                                           "points_per_launch": vol_pts, "share_of_step": vol_ms_max / run_ms_max,
                                           "note": "all volume kernels of one RK stage (interior, PML slabs, "

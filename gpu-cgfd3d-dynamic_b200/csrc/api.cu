@@ -335,6 +335,11 @@ bool late_boxes(const cgfd_solver *s, VolArgs &v) {
   return ok;
 }
 
+// does a small grid's interior and boundary launch leave the fault planes to
+// the late one?  With the surface rows in the shell kind (CGFD_TOP=0) nothing
+// is deferred and the volume launches wait for the split nodes
+bool merged_defers(const cgfd_solver *s) { return !s->isfree || s->nkbox[7] > 0; }
+
 long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = true) {
   const int ip = it % 8;
   const bool tm = s->timing && timed;
@@ -407,9 +412,8 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
   const int nfa = stage_fargs(0, fargs);
   // small grids (merge_points): one launch of all PML kinds and one of the
   // interior box side by side with the fault kernels, then one of the surface
-  // rows and the fault planes beside the fault slabs.  The timed graphs keep
-  // the separate kernels' schedule, in which the interior launch is timed
-  const bool merged = s->merged && !tm;
+  // rows and the fault planes beside the fault slabs
+  const bool merged = s->merged;
   // the volume kernels' arguments of one stage, without boxes
   auto stage_vargs = [&](int stage) {
     const int Lcur = stage == 0 ? LP : (stage == 2 ? LB : LA);
@@ -430,12 +434,15 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
     }
     return v;
   };
+  // external event nodes when captured, so that the events really fire on
+  // every graph replay
+  auto record_timed = [&](cudaEvent_t ev) {
+    if (tm) cudaEventRecordWithFlags(ev, s->stream, cudaEventRecordExternal);
+  };
   auto merged_stage = [&](int stage) {
     const int idir = (kPairs[ip][0] + stage) % 2, jdir = (kPairs[ip][1] + stage) % 2, kdir = (kPairs[ip][2] + stage) % 2;
     VolArgs v = stage_vargs(stage);
-    // with the surface rows in the shell kind (CGFD_TOP=0) nothing is
-    // deferred and the volume launch waits for the split nodes
-    const bool defer = nfa > 0 && (!s->isfree || s->nkbox[7] > 0);
+    const bool defer = nfa > 0 && merged_defers(s);
     if (nfa > 0) {
       if (stage > 0) stage_fargs(stage, fargs);
       cudaEventRecord(s->ev_stage[stage], s->stream);
@@ -459,8 +466,12 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
     }
     volume_boxes(vi, 0, s->kbox[0], s->nkbox[0], false);
     vi.ychunk = s->ychunk;
+    // the timed interval starts behind the forks, which it does not hold up
+    record_timed(s->ev_vol[ip][stage][0]);
     if (vi.nbox > 0) {
+      record_timed(s->ev_int0[ip][stage]);
       launch_volume_interior(vi, idir, jdir, kdir, stage, s->stream);
+      record_timed(s->ev_int[ip][stage]);
       nl++;
     }
     if (vb.nbox > 0) {
@@ -478,6 +489,7 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
       }
     }
     if (nfa > 0) cudaStreamWaitEvent(s->stream, s->ev_postdone[stage], 0);
+    record_timed(s->ev_vol[ip][stage][1]);
   };
   for (int stage = 0; stage < 4; stage++) {
     if (merged) {
@@ -506,10 +518,9 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
         fault_pre(stage, fargs, nfa, s->stream);
       }
     }
-    // external event nodes when captured, so that the events really fire
-    // on every graph replay; the stage interval spans the fork to the join
-    if (tm) cudaEventRecordWithFlags(s->ev_vol[ip][stage][0], s->stream, cudaEventRecordExternal);
-    cudaStream_t st_int = s->stream, st_fault = s->stream, st_pml = s->stream;
+    // the stage interval spans the fork to the join
+    record_timed(s->ev_vol[ip][stage][0]);
+    cudaStream_t st_fault = s->stream, st_pml = s->stream;
     if (br) {
       st_fault = s->aux[0];
       st_pml = s->aux[1];
@@ -578,9 +589,9 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
         if (vk.nbox == 0) continue;
         switch (kind) {
           case 0:
-            if (tm) cudaEventRecordWithFlags(s->ev_int0[ip][stage], st_int, cudaEventRecordExternal);
-            launch_volume_interior(vk, idir, jdir, kdir, mode, st_int);
-            if (tm) cudaEventRecordWithFlags(s->ev_int[ip][stage], st_int, cudaEventRecordExternal);
+            record_timed(s->ev_int0[ip][stage]);
+            launch_volume_interior(vk, idir, jdir, kdir, mode, s->stream);
+            record_timed(s->ev_int[ip][stage]);
             break;
           case 1: launch_volume_shell(vk, idir, jdir, kdir, mode, st_pml); break;
           case 2: launch_volume_face_x(vk, idir, jdir, kdir, mode, st_pml); break;
@@ -611,7 +622,7 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
         cudaStreamWaitEvent(s->stream, s->ev_join[stage][1], 0);
       }
     }
-    if (tm) cudaEventRecordWithFlags(s->ev_vol[ip][stage][1], s->stream, cudaEventRecordExternal);
+    record_timed(s->ev_vol[ip][stage][1]);
   }
   // end of step on the time n+1 level: sponge, then the surface peaks
   // (drv_rk_curv_col.cu:600-613)
@@ -1078,9 +1089,9 @@ int cgfd_upload(const cgfd_setup *su, cgfd_solver **out) {
         }
       }
     }
-    // the fault planes deferred to the PLANE launch (welded nodes of the
-    // grown split box; the split nodes belong to the fault kernels)
-    if (s->pre_overlap)
+    // the fault planes deferred to the PLANE or the late launch (welded nodes
+    // of the grown split box; the split nodes belong to the fault kernels)
+    if (s->merged ? merged_defers(s) : s->pre_overlap)
       for (size_t f = 0; f < H.faults.size(); f++) {
         const FaultState &F = s->faults[f];
         const int i = H.faults[f].i0 - NG;

@@ -267,10 +267,11 @@ int cgfd_last_launches(const cgfd_solver *s, long long *launches);
 
 /* 1: time every volume-stage launch with CUDA events on the solver's
  * stream (cgfd_run reads each step's events 8 steps later, so the host
- * never waits on the step in flight); 0: off (default).  Switching builds
- * the step graphs of the new mode if they do not exist yet (cgfd_upload
- * builds those of the default mode), so that no graph is captured or
- * instantiated inside a run. */
+ * never waits on the step in flight); 0: off (default).  The events add no
+ * launch and change no order: what is timed is the step that runs without
+ * them.  Switching builds the step graphs of the new mode if they do not
+ * exist yet (cgfd_upload builds those of the default mode), so that no graph
+ * is captured or instantiated inside a run. */
 int cgfd_set_timing(cgfd_solver *s, int on);
 /* Device time of the last cgfd_run (events on the solver's stream at its
  * start and end) and, with timing on, the summed duration and count of its
@@ -280,7 +281,9 @@ int cgfd_last_timing(const cgfd_solver *s, double *run_ms, double *volume_ms,
 /* Per-kernel detail of the last cgfd_run with timing on (no counterpart in
  * the reference; instrumentation for roofline figures).  which = 0: the
  * volume stage (all volume kernels of one RK stage); which = 1: the
- * interior-box kernel alone.  ms: summed device time of the timed launches;
+ * interior-box kernel alone.  ms: summed device time of the timed launches,
+ * each from its start to its end whatever runs beside it (the fault kernels;
+ * on small grids, whose boundary kinds run in one launch, that one too);
  * launches: their number; points: grid points one launch updates. */
 int cgfd_last_kernel_timing(const cgfd_solver *s, int which, double *ms,
                             long long *launches, long long *points);

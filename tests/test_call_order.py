@@ -230,3 +230,54 @@ def test_launch_counts_are_those_of_the_schedule_that_ran(recording, monkeypatch
         check(lambda: a.run(9), [a])
         check(lambda: b.run(9), [b])
     ens.close()
+
+
+@pytest.mark.parametrize("free_surface", [0, 1])
+def test_timing_keeps_the_schedule(recording, free_surface):
+    """cgfd_set_timing adds events to a step, no launch and no order: what it
+    times is the step that runs without it."""
+    from cgfd import Solver
+    p = inputs.small_planar(nt=20, free_surface=free_surface)
+    s = Solver(p, lib=recording)
+
+    def graphs():
+        # a capture's launches with their streams, and its forks and joins
+        out, lines = [], None
+        external = set()
+        for o in operations(recording):
+            if o[0] == "begin":
+                lines = []
+            elif o[0] == "end":
+                out.append(lines)
+                lines = None
+            elif lines is not None and not (o[0] == "record" and o[3] == "1"):
+                lines.append(o)
+            elif lines is not None:
+                external.add(o[2])
+        return out, external
+
+    plain, none = graphs()
+    s.set_timing(True)
+    timed, external = graphs()
+    assert len(plain) == len(timed) == 8 and not none
+    assert any("k_volume_all" in o[2] for o in plain[0] if o[0] == "launch")
+    assert timed == plain
+    # four events a stage, of which every step has its own
+    assert len(external) == 8 * 4 * 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("free_surface", [0, 1])
+def test_timed_run_is_the_untimed_one(cgfd_lib, free_surface):
+    from cgfd import Solver, WAVE_COMPONENTS
+    a, b = (Solver(inputs.small_planar(nt=20, free_surface=free_surface)) for _ in range(2))
+    b.set_timing(True)
+    for s in (a, b):
+        s.run(17)
+    assert a.last_launches() == b.last_launches()
+    run_ms, vol_ms, vol_n = b.last_timing()
+    int_ms, int_n, _ = b.kernel_timing(1)
+    assert vol_n == int_n == 4 * 17 and 0 < int_ms <= vol_ms <= run_ms
+    for c in WAVE_COMPONENTS:
+        assert np.array_equal(a.wavefield(c), b.wavefield(c)), c
+    assert np.array_equal(a.fault_all(), b.fault_all())
