@@ -36,7 +36,7 @@ void launch_volume_edge(const VolArgs &a, int idir, int jdir, int kdir, int mode
 void launch_volume_plane(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st);
 void launch_volume_top(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaStream_t st);
 int launch_fault_pre(const FaultArgs &a, const StationArgs *rec, cudaStream_t st);
-int launch_fault_post(const FaultArgs &a, cudaStream_t st);
+int launch_fault_post(const FaultArgs &a, bool behind_fault, cudaStream_t st);
 cudaError_t noalloc_scratch_address(real **p);
 void launch_align(const real *rows, real *out, long sc, cudaStream_t st);
 void launch_record(const StationArgs &a, cudaStream_t st);
@@ -354,6 +354,13 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
   auto fault_pre = [&](int stage, const FaultArgs *fa, int n, cudaStream_t st) {
     for (int f = 0; f < n; f++) nl += launch_fault_pre(fa[f], rec && stage == 0 && f == 0 ? &sa : nullptr, st);
   };
+  auto fault_post = [&](const FaultArgs *fa, int n, bool behind_fault, cudaStream_t st) {
+    for (int f = 0; f < n; f++) {
+      const int l = launch_fault_post(fa[f], behind_fault, st);
+      nl += l;
+      behind_fault |= l > 0;
+    }
+  };
   // the fault kernels' arguments of one stage
   auto stage_fargs = [&](int stage, FaultArgs *fa) {
     const int idir = (kPairs[ip][0] + stage) % 2, jdir = (kPairs[ip][1] + stage) % 2, kdir = (kPairs[ip][2] + stage) % 2;
@@ -449,7 +456,7 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
       cudaStreamWaitEvent(s->aux[0], s->ev_stage[stage], 0);
       fault_pre(stage, fargs, nfa, s->aux[0]);
       cudaEventRecord(s->ev_predone[stage], s->aux[0]);
-      for (int f = 0; f < nfa; f++) nl += launch_fault_post(fargs[f], s->aux[0]);
+      fault_post(fargs, nfa, true, s->aux[0]);
       cudaEventRecord(s->ev_postdone[stage], s->aux[0]);
       if (!defer) cudaStreamWaitEvent(s->stream, s->ev_predone[stage], 0);
     }
@@ -511,7 +518,7 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
         fault_pre(stage, fargs, nfa, s->aux[0]);
         cudaEventRecord(s->ev_predone[stage], s->aux[0]);
         if (pe2) {
-          for (int f = 0; f < nfa; f++) nl += launch_fault_post(fargs[f], s->aux[0]);
+          fault_post(fargs, nfa, true, s->aux[0]);
           cudaEventRecord(s->ev_postdone[stage], s->aux[0]);
         }
       } else {
@@ -528,8 +535,7 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
       cudaStreamWaitEvent(st_fault, s->ev_fork[stage], 0);
       cudaStreamWaitEvent(st_pml, s->ev_fork[stage], 0);
     }
-    if (!br2)
-      for (int f = 0; f < nfa; f++) nl += launch_fault_post(fargs[f], st_fault);
+    if (!br2) fault_post(fargs, nfa, !br && !tm, st_fault);
     VolArgs vs = stage_vargs(stage);
     vs.defer_i0 = ov ? 1 : 0;
     {
@@ -553,7 +559,7 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
           if (br3) cudaStreamWaitEvent(s->aux[1], s->ev_fork[stage], 0);
           if (!pe2) {
             cudaStreamWaitEvent(st_fault, s->ev_fork[stage], 0);
-            for (int f = 0; f < nfa; f++) nl += launch_fault_post(fargs[f], st_fault);
+            fault_post(fargs, nfa, false, st_fault);
             if (ov) cudaEventRecord(s->ev_postdone[stage], st_fault);
           }
         }
@@ -570,7 +576,7 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
             // and their stencils stay clear of the fault neighbourhood), and
             // no kernel of this stage reads or writes the next stage's
             // output or end level there
-            for (int f = 0; f < nfa; f++) nl += launch_fault_post(fnext[f], st_fault);
+            fault_post(fnext, nfa, true, st_fault);
             cudaEventRecord(s->ev_postdone[stage + 1], st_fault);
           }
         }

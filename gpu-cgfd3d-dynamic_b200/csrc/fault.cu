@@ -861,11 +861,16 @@ int launch_fault_pre(const FaultArgs &a, const StationArgs *rec, cudaStream_t st
 }
 
 // second part: the slab points around the split nodes; independent of the
-// volume kernels of the same stage (disjoint outputs, shared read-only input)
-int launch_fault_post(const FaultArgs &a, cudaStream_t st) {
+// volume kernels of the same stage (disjoint outputs, shared read-only input).
+// behind_fault: the operation ahead in the stream is a fault kernel, whose end
+// the launch may overlap; behind an event wait or a timing event it is an
+// ordinary launch
+int launch_fault_post(const FaultArgs &a, bool behind_fault, cudaStream_t st) {
   if (a.nj <= 0 || a.nk <= 0) return 0;
   const long nslab = (long)a.nj * a.nk * 6;
-  launch_after(k_fault_slab, dim3((unsigned)((nslab + kSlabPoints - 1) / kSlabPoints)), dim3(kSlabPoints, 2), st, a);
+  const dim3 grd((unsigned)((nslab + kSlabPoints - 1) / kSlabPoints)), blk(kSlabPoints, 2);
+  if (behind_fault) launch_after(k_fault_slab, grd, blk, st, a);
+  else k_fault_slab<<<grd, blk, 0, st>>>(a);
   return 1;
 }
 

@@ -281,3 +281,58 @@ def test_timed_run_is_the_untimed_one(cgfd_lib, free_surface):
     for c in WAVE_COMPONENTS:
         assert np.array_equal(a.wavefield(c), b.wavefield(c)), c
     assert np.array_equal(a.fault_all(), b.fault_all())
+
+
+SCHEDULES = [{}, {"CGFD_MERGED": "0"}, {"CGFD_BRANCHES": "0"}, {"CGFD_BRANCHES": "1"}, {"CGFD_BRANCHES": "2"},
+             {"CGFD_PRE_OVERLAP": "0"}, {"CGFD_POST_EARLY": "0"}, {"CGFD_PRE_EARLY": "0"},
+             {"CGFD_TOP": "0"}]
+
+
+@pytest.mark.parametrize("env", SCHEDULES, ids=lambda e: ",".join(f"{k}={v}" for k, v in e.items()) or "default")
+def test_dependent_launches_follow_their_kernel(recording, monkeypatch, env):
+    """A programmatic dependent launch starts beside the operation ahead of it
+    in its stream; it is used only where that is the fault kernel it was
+    written to run beside, never behind an event wait or a timing event."""
+    from cgfd import Solver
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    ahead_of = {"k_fault_split": {"k_fault_pre"}, "k_fault_slab": {"k_fault_split", "k_fault_slab"}}
+    for p in (clear_of_the_pml(), closed_box(), inputs.two_faults(nt=20)):
+        s = Solver(p, lib=recording)
+        s.set_timing(True)
+        s.set_timing(False)
+        try:
+            s.run_noalloc(1)
+        except Exception as e:      # free surface: nothing counts the steps here
+            assert "counter" in str(e)
+        last, dependent = {}, set()
+        for op, st, *rest in operations(recording):
+            if op == "launch":
+                name = kernel(rest[0])
+                if rest[-1] == "1":
+                    assert last[st] in ahead_of[name], (name, last[st])
+                    dependent.add(name)
+                last[st] = name
+            elif op != "record" or rest[1] == "1":
+                last[st] = op
+        assert "k_fault_split" in dependent
+        s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("env", SCHEDULES, ids=lambda e: ",".join(f"{k}={v}" for k, v in e.items()) or "default")
+def test_timed_schedules_agree(cgfd_lib, monkeypatch, env):
+    """Every schedule with timing on (its events lie among the launches) is
+    the untimed one bit for bit."""
+    from cgfd import Solver, WAVE_COMPONENTS
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    for p in (clear_of_the_pml(), inputs.two_faults(nt=20)):
+        a, b = Solver(p), Solver(p)
+        b.set_timing(True)
+        for s in (a, b):
+            s.run(17)
+        for c in WAVE_COMPONENTS:
+            assert np.array_equal(a.wavefield(c), b.wavefield(c)), c
+        for f in range(p.num_faults):
+            assert np.array_equal(a.fault_all(f), b.fault_all(f)), f
