@@ -771,9 +771,11 @@ static int build_graphs(cgfd_solver *s);
 // take): the first stage's interior launch is timed for a few chunk sizes
 // on the solver's state at upload, which is all zero, so the launches write
 // zeros where zeros are and change nothing.  The fastest size is kept per
-// device and interior box, so later solvers of the same shape reuse it.
+// device, interior box, row pitch and kernel (aligned or general: 32 or 48
+// bytes of metric and medium a point), so later solvers of the same shape
+// reuse it.
 static std::mutex g_tune_mu;
-static std::map<std::array<int, 4>, int> g_tune;
+static std::map<std::array<int, 6>, int> g_tune;
 
 static cudaError_t tune_ychunk(cgfd_solver *s) {
   if (s->nkbox[0] == 0) return cudaSuccess;
@@ -781,7 +783,7 @@ static cudaError_t tune_ychunk(cgfd_solver *s) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const std::array<int, 4> key = { dev, B[1] - B[0] + 1, B[3] - B[2] + 1, B[5] - B[4] + 1 };
+  const std::array<int, 6> key = { dev, B[1] - B[0] + 1, B[3] - B[2] + 1, B[5] - B[4] + 1, (int)s->g.sy, s->g.al };
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto f = g_tune.find(key);

@@ -336,3 +336,24 @@ def test_timed_schedules_agree(cgfd_lib, monkeypatch, env):
             assert np.array_equal(a.wavefield(c), b.wavefield(c)), c
         for f in range(p.num_faults):
             assert np.array_equal(a.fault_all(f), b.fault_all(f)), f
+
+
+def test_chunk_choice_is_kept_per_kernel(recording, monkeypatch):
+    """The interior kernel's y chunk is timed once per kernel and grid shape: a
+    solver that runs the general kernel does not take over what was fastest
+    for the aligned one on an interior box of the same extents."""
+    from cgfd import Solver
+    p = inputs.small_planar(nt=20, ni=38, nj=58)
+
+    def timed():
+        operations(recording)
+        Solver(p, lib=recording).close()
+        ops = operations(recording)
+        first = next(n for n, o in enumerate(ops) if o[0] == "begin")
+        return sum(o[0] == "launch" and kernel(o[2]) == "k_volume 0" for o in ops[:first])
+
+    assert timed() > 0 and timed() == 0
+    monkeypatch.setenv("CGFD_ALIGNED", "0")
+    assert timed() > 0 and timed() == 0
+    monkeypatch.delenv("CGFD_ALIGNED")
+    assert timed() == 0
