@@ -1076,10 +1076,11 @@ int cgfd_upload(const cgfd_setup *su, cgfd_solver **out) {
     // 1200x600x400 best at 128-192 rows, 600x300x240 at its whole plane)
     {
       const long row_bytes = (long)std::max(1, ihi - ilo + 1) * kTileY * 36;
-      s->ychunk = (int)std::max(4L, (24L << 20) / (8 * row_bytes));
+      s->ychunk = (int)std::max(32L / kTileY, (24L << 20) / (8 * row_bytes));
     }
+    // the switch counts 8 rows, whatever the tiles' height
     const char *yc = std::getenv("CGFD_INTERIOR_YCHUNK");
-    if (yc && std::atoi(yc) > 0) s->ychunk = std::atoi(yc);
+    if (yc && std::atoi(yc) > 0) s->ychunk = (int)std::min(8L * std::atoi(yc) / kTileY, 65535L);
     s->ychunk = std::min(s->ychunk, std::max(1, (jhi - jlo + kTileY) / kTileY));
     // points one interior launch / one volume stage updates: the split-node
     // slabs belong to the fault kernels

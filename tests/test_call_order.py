@@ -357,3 +357,20 @@ def test_chunk_choice_is_kept_per_kernel(recording, monkeypatch):
     assert timed() > 0 and timed() == 0
     monkeypatch.delenv("CGFD_ALIGNED")
     assert timed() == 0
+
+
+@pytest.mark.parametrize("n", [1, 2, 100])
+def test_chunk_switch_counts_eight_rows(recording, monkeypatch, n):
+    """CGFD_INTERIOR_YCHUNK=n asks for chunks of 8 n rows whatever the height
+    of the kernel's tiles (so its grid's z extent, which is limited to 65535,
+    does not grow when the tiles get lower)."""
+    from cgfd import Solver
+    p = inputs.small_planar(nt=20, nj=61)
+    rows, planes = 61 - 2 * 6, 32 - 6 - 4
+    monkeypatch.setenv("CGFD_INTERIOR_YCHUNK", str(n))
+    operations(recording)
+    Solver(p, lib=recording).close()
+    grid = next([int(v) for v in o[3:6]] for o in operations(recording) if o[0] == "launch" and kernel(o[2]) == "k_volume 0")
+    tiles = -(-rows // 4)
+    chunk = min(2 * n, tiles)
+    assert grid[1:] == [chunk, planes * -(-tiles // chunk)]
