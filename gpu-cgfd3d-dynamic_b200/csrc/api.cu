@@ -163,14 +163,14 @@ struct cgfd_setup {
 namespace {
 
 // host floats (the set-up's arrays) to device values of type real on the
-// solver's stream; the double build widens them on the host first and
-// copies synchronously
+// solver's stream; the double build widens them on the host first and waits
+// for its copy
 cudaError_t to_device(real *dst, const float *src, size_t n, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
 #ifdef CGFD_FP64
   std::vector<double> wide(src, src + n);
-  cudaError_t e = cudaStreamSynchronize(st);
-  return e == cudaSuccess ? cudaMemcpy(dst, wide.data(), n * sizeof(double), cudaMemcpyHostToDevice) : e;
+  cudaError_t e = cudaMemcpyAsync(dst, wide.data(), n * sizeof(double), cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
 #else
   return cudaMemcpyAsync(dst, src, n * sizeof(float), cudaMemcpyHostToDevice, st);
 #endif
@@ -1724,12 +1724,17 @@ int cgfd_restore(cgfd_solver *s, const void *buf, unsigned long long bytes) {
   p += sizeof(int);
   if (it < 0) return fail(CGFD_ERR_ARG, "corrupt checkpoint");
   s->it = it;   // sets the level parity before the parts are placed
+  // on the solver's stream: a blocking copy of pageable memory may return
+  // before the device has its last part, and orders nothing on this stream
+  cudaError_t e = cudaSuccess;
   for (auto &q : state_parts(s)) {
-    cudaError_t e = cudaMemcpy(q.first, p, q.second, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return cuda_fail(e, "restore");
+    e = cudaMemcpyAsync(q.first, p, q.second, cudaMemcpyHostToDevice, s->stream);
+    if (e != cudaSuccess) break;
     p += q.second;
   }
-  return CGFD_OK;
+  const cudaError_t w = cudaStreamSynchronize(s->stream);
+  if (e == cudaSuccess) e = w;
+  return e == cudaSuccess ? CGFD_OK : cuda_fail(e, "restore");
 }
 
 int cgfd_last_launches(const cgfd_solver *s, long long *n) {

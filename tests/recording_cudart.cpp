@@ -8,7 +8,7 @@
 // The log is one line per operation, "op stream rest":
 //   launch S name gx gy gz pdl   kernel launch (pdl 1: programmatic dependent)
 //   set S bytes / copy S bytes   asynchronous clear / copy
-//   blockcopy 0 bytes            cudaMemcpy (the default stream)
+//   blockcopy 0 bytes in|out     cudaMemcpy (the default stream), to or from the device
 //   record S event external      wait S event
 //   graph S exec                 sync S (the host waits for stream S)
 //   begin S / end S exec         capture (what lies between is in the graph)
@@ -90,7 +90,11 @@ cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { return alloc(p, 
 cudaError_t cudaMallocHost(void **p, size_t n) { return alloc(p, n); }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { std::free(p); return cudaSuccess; }
 cudaError_t cudaFreeHost(void *p) { std::free(p); return cudaSuccess; }
-cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); log("blockcopy", nullptr, std::to_string(n)); return cudaSuccess; }
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind k) {
+  std::memcpy(d, s, n);
+  log("blockcopy", nullptr, std::to_string(n) + (k == cudaMemcpyDeviceToHost ? " out" : " in"));
+  return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) { std::memcpy(d, s, n); log("copy", st, std::to_string(n)); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t st) { std::memset(d, v, n); log("set", st, std::to_string(n)); return cudaSuccess; }
 

@@ -17,19 +17,27 @@ import inputs
 from conftest import PKG, TESTS
 
 
-@pytest.fixture(scope="module")
-def recording(cgfd_lib, tmp_path_factory):
-    """The float library on the recording runtime."""
+def on_recording_runtime(d, kind):
+    """The library of the build's *.cu{kind}.o objects on the recording runtime."""
     import cgfd
-    d = tmp_path_factory.mktemp("recording")
     obj, lib = str(d / "recording_cudart.o"), str(d / "libcgfd_recording.so")
     subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-I/usr/local/cuda/include", "-c",
                            os.path.join(TESTS, "recording_cudart.cpp"), "-o", obj])
-    built = sorted(glob.glob(os.path.join(PKG, "_build", "*.cu.o"))) + [os.path.join(PKG, "_build", "setup.cpp.o")]
+    built = sorted(glob.glob(os.path.join(PKG, "_build", f"*.cu{kind}.o"))) + [os.path.join(PKG, "_build", "setup.cpp.o")]
     subprocess.check_call(["g++", "-shared", "-Wl,-Bsymbolic", "-o", lib] + built + [obj, "-lgomp"])
     r = cgfd.load_library(lib)
     r.recording_log.restype = ctypes.c_char_p
     return r
+
+
+@pytest.fixture(scope="module")
+def recording(cgfd_lib, tmp_path_factory):
+    return on_recording_runtime(tmp_path_factory.mktemp("recording"), "")
+
+
+@pytest.fixture(scope="module")
+def recording64(cgfd_lib, tmp_path_factory):
+    return on_recording_runtime(tmp_path_factory.mktemp("recording64"), "64")
 
 
 def operations(lib, clear=True):
@@ -374,3 +382,29 @@ def test_chunk_switch_counts_eight_rows(recording, monkeypatch, n):
     tiles = -(-rows // 4)
     chunk = min(2 * n, tiles)
     assert grid[1:] == [chunk, planes * -(-tiles // chunk)]
+
+
+@pytest.mark.parametrize("double", [False, True])
+def test_writes_to_the_device_follow_the_solvers_stream(recording, recording64, double):
+    """The blocking copy of pageable memory may return before the device has
+    all of it, and orders nothing on the solver's stream: a state or a
+    wavefield that is put in place goes by that stream, and is waited for."""
+    from cgfd import Solver
+    lib = recording64 if double else recording
+    operations(lib)
+    s = Solver(closed_box(), lib=lib)
+    s.run(1)
+    calls = [operations(lib)]
+    buf = s.checkpoint()
+    operations(lib)
+    s.restore(buf)
+    calls.append(operations(lib))
+    s.set_wavefield("Vx", np.zeros((s.prob.nk, s.prob.nj, s.prob.ni), np.float32))
+    calls.append(operations(lib))
+    for ops in calls:
+        assert not any(o[0] == "blockcopy" and o[3] == "in" for o in ops)
+        assert any(o[0] == "copy" for o in ops)
+    for ops in calls[1:]:
+        streams = {o[1] for o in ops if o[0] == "copy"}
+        assert len(streams) == 1 and ops[-1] == ("sync", streams.pop())
+    s.close()
