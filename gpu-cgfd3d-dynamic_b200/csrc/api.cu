@@ -85,7 +85,7 @@ struct cgfd_solver {
   int imethod = 2, isfree = 0;
   float dt = 0.f, dtmax = 0.f;
   real *w[4] = {};                      // storage slots of the 4 levels
-  real *coef = nullptr, *free_mat = nullptr;    // packed metric and medium (13 scmp values)
+  real *coef = nullptr, *free_mat = nullptr;    // packed metric and medium (13 scmp values, 9 on aligned grids), free-surface matrices
   real *abl_E = nullptr;                // sponge masks [nx | ny | nz]
   SpongeArgs sponge{};                  // sponge blocks (w set per step)
   real *pg = nullptr, *dis = nullptr;   // surface peaks [15][nj][ni], displacement [3][nj][ni]
@@ -274,11 +274,6 @@ size_t trac_slices(const cgfd_solver *s, size_t *off) {
   return n;
 }
 
-// enqueue one time step (graph capture or direct launches); trac: one
-// traction scratch to use instead of each fault's own (cgfd_run_noalloc),
-// split into one slice per fault because the first fault kernels of every
-// fault run before the later ones of any fault; timed: whether the
-// solver's timing events may be recorded; returns the number of launches
 // the fault planes of a volume launch: x = i0 of each fault, its split-node
 // flags and the deferred box (the split box grown by 3 nodes, empty when the
 // fault has no split node)
@@ -299,11 +294,19 @@ void fault_planes(const cgfd_solver *s, VolArgs &v) {
 // ones are bound by the chain of dependent launches and by launches that do
 // not fill the GPU, large ones by bytes, where each kind's own code and
 // register count pay.  Without a free surface there are two kinds fewer to
-// chain.  Measured, step apart / together: free surface 0.06 M points
-// 167 / 102 us, 0.24 M (no fault) 193 / 93, 0.46 M 320 / 241, 0.91 M 399 / 329,
-// 1.28 M 453 / 403, 1.94 M 564 / 505, 3.39 M 804 / 800, 5.24 M 1157 / 1159;
-// PML on all faces 0.06 M 119 / 95, 0.14 M 145 / 119, 0.27 M 167 / 157,
-// 0.39 M 201 / 203, 1.28 M 391 / 406, without a fault 0.91 M 254 / 229.
+// chain.  Measured, step apart / together in us (shapes 36x56x32, 64x96x50,
+// 64x128x64, 96x140x72, 100x160x80, 128x160x90, 128x200x100, 160x200x110,
+// 160x256x128; faces of 5 to 10 layers):
+//   points            0.06M    0.31M    0.52M    0.97M    1.28M    1.84M    2.56M    3.52M    5.24M
+//   free, fault      159/97  245/156  324/255  377/357  437/435  524/523  666/677  835/849 1161/1189
+//   free, 20 layers     -        -    347/313  426/411  489/490  578/600  735/756  914/950 1266/1326
+//   free, no fault   125/56   194/92  249/153  311/240  363/299  441/377  562/513  684/647   969/921
+//   closed, fault    103/87  165/150  242/255  317/351  379/431  466/531  631/685  778/841 1141/1210
+//   closed, none      70/45   124/94  173/166  255/260  311/324  402/420  529/547  682/693   955/962
+// (long and flat shapes lie between, 40x400x200 with a fault 1279/1238.)  Two
+// numbers for the two sides of the free surface do not fit every row: with
+// thick faces the free surface's line lies 1 M too high (2 to 4% of those
+// steps), without a fault it could lie above 5 M (5%).
 long long merge_points(const cgfd_solver *s) {
   return s->isfree ? 3'500'000 : (s->faults.empty() ? 1'000'000 : 300'000);
 }
@@ -340,6 +343,11 @@ bool late_boxes(const cgfd_solver *s, VolArgs &v) {
 // is deferred and the volume launches wait for the split nodes
 bool merged_defers(const cgfd_solver *s) { return !s->isfree || s->nkbox[7] > 0; }
 
+// enqueue one time step (graph capture or direct launches); trac: one
+// traction scratch to use instead of each fault's own (cgfd_run_noalloc),
+// split into one slice per fault because the first fault kernels of every
+// fault run before the later ones of any fault; timed: whether the
+// solver's timing events may be recorded; returns the number of launches
 long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed = true) {
   const int ip = it % 8;
   const bool tm = s->timing && timed;
@@ -540,8 +548,7 @@ long long enqueue_step(cgfd_solver *s, int it, real *trac = nullptr, bool timed 
     vs.defer_i0 = ov ? 1 : 0;
     {
       // interior box, single-direction PML slabs, generic shell
-      const int kind0 = 0;
-      for (int kind = kind0; kind < 6; kind++) {
+      for (int kind = 0; kind < 6; kind++) {
         if (kind == 1 && ov) {
           // the fault planes x = i0 once the stage's first fault kernels
           // (which refresh the split nodes there) are done
@@ -974,10 +981,12 @@ int cgfd_upload(const cgfd_setup *su, cgfd_solver **out) {
     // surface rows over the interior box's x extent are cut the same way,
     // their leftover columns going to the generic edge and shell kernels.
     // The PML kernels take about 1.8 times the interior kernel's time per
-    // point, so more columns stay where they are: measured per step, all
-    // joining / staying: 6 columns (240 wide) 2.754 / 2.814 ms, 14 (100 wide)
-    // 0.512 / 0.507, 15 (101) 0.457 / 0.437, 24 (120) 0.518 / 0.488, 30 (200)
-    // 2.339 / 2.221.
+    // point, so more columns stay where they are.  Measured, step joining over
+    // staying, at about 0.4, 1.3, 3.7 and 11 M points: faces of 10 layers
+    // 2 columns 0.92-0.98, 8 0.96-0.98, 10 0.95-0.98, 12 0.97-0.99, 14 0.99-1.02,
+    // 16 0.99-1.04, 20 1.00-1.05; of 20 layers 2 columns 0.93-0.97, 8 0.95-0.98,
+    // 10 0.95-0.99, 12 1.00-1.05, 14 and more 1.00-1.06.  The slab's own width
+    // decides from 12 on; 9 to 11 columns could join as well (2 to 5%).
     constexpr int kMaxLeftover = 8;
     int iha = ihi;
     {

@@ -93,7 +93,8 @@ __device__ __forceinline__ real rk_put(int mode, real ca, real cb, real u0, real
 }
 
 // Programmatic dependent launch: a kernel launched with launch_after() may
-// start before the one ahead of it in its stream has ended.  after_previous()
+// start before the one ahead of it in its stream has ended (in an ordinary
+// launch both instructions do nothing).  after_previous()
 // waits for that one's end (and its writes), let_next_start() lets the next
 // one's blocks in.  The split-node kernel reads its node's own values while
 // the first fault kernel runs, the slab kernel forms its stress right-hand

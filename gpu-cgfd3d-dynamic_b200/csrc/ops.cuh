@@ -58,11 +58,8 @@ enum { LP = 0, LA = 1, LB = 2, LE = 3 };
 // 0.515 on 100x160x80.
 enum { RK_FIRST = 0, RK_SECOND = 1, RK_THIRD = 2, RK_LAST = 3 };
 
-// does a stage of this mode read the time-n level / write the next input /
-// write the fourth level
+// does a stage of this mode read the time-n level?
 __host__ __device__ constexpr bool rk_reads_pre(int mode) { return mode == RK_SECOND || mode == RK_THIRD; }
-__host__ __device__ constexpr bool rk_writes_out(int mode) { return mode != RK_LAST; }
-__host__ __device__ constexpr bool rk_writes_end(int mode) { return mode == RK_SECOND || mode == RK_LAST; }
 // next stage input from the level it starts from (u0) and its increment
 __device__ __forceinline__ real rk_out(real u0, real inc) { return u0 + inc; }
 // V of the second stage: cur = u1, inc = u2 - u0

@@ -31,7 +31,13 @@ struct FaultHost {
 
 // An off-axis metric entry this far below its row's own is the rounding of
 // the coordinate differences that should cancel (they leave up to 2^-43 on
-// the workloads); its products are below 2^-16 of a float's last bit.
+// the workloads).  The bound is one of the entries: a product of such an entry
+// may still be the larger one where the derivative that the kept entry
+// multiplies is near zero.  Measured on what they change: relative L2 error
+// of each component against 64 bits with these entries and without them, 20
+// steps of 0.24 M and 1.28 M points from random and from one-component states
+// (planar, hills, faultless, buried, sponge): ratio 1.000 on average, 1.003 at
+// most, at errors of 3e-7 to 9e-7.
 constexpr float kAligned = 1.0f / (1ll << 40);
 
 struct HostSetup {

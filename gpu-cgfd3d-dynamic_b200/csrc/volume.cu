@@ -101,8 +101,9 @@ __device__ __forceinline__ Taps taps_at(const real *w, long sc, unsigned p) {
 // sm_100 one fma.rn.f32x2 does two multiply-adds, each rounded as the
 // scalar one, so the 27 derivatives of a point take 75 instructions instead
 // of 135 (interior launch of 30.0 M points with waves everywhere, where the
-// GPU sits at its 1000 W cap: 1.089 -> 1.058 ms; from 16-24 bytes of spills to
-// none at 64 registers).
+// GPU sits at its 1000 W cap: 1.089 -> 1.058 ms).  At 64 registers 17 of the 64
+// interior instantiations spill 4-16 bytes, 7 of them the aligned ones of
+// stage 2, which writes two levels.
 #ifdef CGFD_FP64
 typedef double2 real2;
 __device__ __forceinline__ real2 mul2(real c, real2 x) { return make_double2(c * x.x, c * x.y); }
@@ -696,7 +697,9 @@ __global__ void __launch_bounds__(BX * BY, KIND == INTERIOR || KIND == PLANE ? C
 // every kind in one launch, each block the kind of its box (merge_points in
 // api.cu says when).  6 blocks per SM as the boundary kinds have them alone;
 // 5: 105 us per step of 36x56x32 and 419 of 101x163x77, 8: 116 and 433, 6: 107
-// and 420.
+// and 420.  One register budget (80) for seven bodies: every instantiation
+// spills, 4-132 bytes on aligned grids and 36-196 on others, the second
+// stage's the most.
 template <int ID, int JD, int KD, int MODE, bool AL>
 __global__ void __launch_bounds__(BX * BY, CGFD_LB_ALL) k_volume_all(const __grid_constant__ VolArgs a) {
   const int b = box_of_block(a);
@@ -767,9 +770,10 @@ void launch_kind(const VolArgs &a, int idir, int jdir, int kdir, int mode, cudaS
 }  // namespace
 
 // This file is compiled once per kernel kind (CGFD_VOLUME_KIND = 0..7, set
-// by the build) so that the 32 instantiations of each kind build in
-// parallel, and once per operator triple for the kernels that hold every
-// kind (8..15); unit 0 also holds the host helpers.
+// by the build) so that the 64 instantiations of each kind (32 in the double
+// build, which has no aligned ones) build in parallel, and once per operator
+// triple for the kernels that hold every kind (8..15); unit 0 also holds the
+// host helpers.
 #ifndef CGFD_VOLUME_KIND
 #define CGFD_VOLUME_KIND 0
 #endif
