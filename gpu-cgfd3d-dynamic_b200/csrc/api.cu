@@ -781,6 +781,7 @@ static int build_graphs(cgfd_solver *s);
 // device, interior box, row pitch and kernel (aligned or general: 32 or 48
 // bytes of metric and medium a point), so later solvers of the same shape
 // reuse it.
+constexpr int kMaxChunk = 65535;   // tiles: the interior launch's y extent
 static std::mutex g_tune_mu;
 static std::map<std::array<int, 6>, int> g_tune;
 
@@ -811,7 +812,7 @@ static cudaError_t tune_ychunk(cgfd_solver *s) {
   float best_ms = 1e30f;
   std::vector<int> cand;
   for (int c : { 16, 32, 64, 128, ntiles }) {
-    c = std::max(1, std::min(c, ntiles));
+    c = std::max(1, std::min({ c, ntiles, kMaxChunk }));
     if (std::find(cand.begin(), cand.end(), c) == cand.end()) cand.push_back(c);
   }
   for (int c : cand) {
@@ -1089,7 +1090,7 @@ int cgfd_upload(const cgfd_setup *su, cgfd_solver **out) {
     }
     // the switch counts 8 rows, whatever the tiles' height
     const char *yc = std::getenv("CGFD_INTERIOR_YCHUNK");
-    if (yc && std::atoi(yc) > 0) s->ychunk = (int)std::min(8L * std::atoi(yc) / kTileY, 65535L);
+    if (yc && std::atoi(yc) > 0) s->ychunk = (int)std::min(8L * std::atoi(yc) / kTileY, (long)kMaxChunk);
     s->ychunk = std::min(s->ychunk, std::max(1, (jhi - jlo + kTileY) / kTileY));
     // points one interior launch / one volume stage updates: the split-node
     // slabs belong to the fault kernels
